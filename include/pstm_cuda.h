@@ -144,7 +144,7 @@ void pstm_cuda_destroy(void *ctx);
 /* Migrate one tile, device pointers, asynchronous on `stream` (a
  * cudaStream_t; NULL = the context's stream; pass cudaStreamLegacy, 0x1, for
  * the legacy default stream).  Calls on one context must not overlap on the
- * device: the context's per-launch tables are reused by the next call.  Replaces
+ * device: the context's error word and work lists are reused by the next call.  Replaces
  * MigrationKernel.migrate_tile, base.py:305-313;
  * OptimizedNumbaKernel.migrate_tile, numba_cpu_optimized.py:545-626;
  * CompiledMetalKernel.migrate_tile[_curved_ray/_vti], metal_compiled.py:567,1275,1456. */
@@ -157,10 +157,8 @@ int32_t pstm_cuda_migrate_tile_dev(void *ctx, const pstm_traces_desc *traces,
  * runs[2i] .. runs[2i+1] - 1, ascending and disjoint, inside [0, n_traces).
  * The result is that of pstm_cuda_migrate_tile_dev on the concatenation of the
  * ranges, up to the order of floating-point additions, without copying the
- * ranges together: geometry is packed for the span of the runs and one
- * persistent launch takes (run segment, pillar block, time block) items that
- * add into the image and fold atomically (non-linear interpolation: one
- * migration per run).  A panel sorted by midpoint (pstm_b200.spatial) gives
+ * ranges together: the CTAs of one launch walk the ranges (non-linear
+ * interpolation: one migration per run).  A panel sorted by midpoint (pstm_b200.spatial) gives
  * each output tile's traces as a few such runs.  Device pointers;
  * asynchronous on `stream` as pstm_cuda_migrate_tile_dev.  Replaces the
  * executor's per-tile trace query and gather, SpatialIndex.query_traces_for_tile
@@ -174,12 +172,11 @@ int32_t pstm_cuda_migrate_tile_runs_dev(void *ctx, const pstm_traces_desc *trace
 /* The trace-centric (scatter) schedule of a migration: instead of every tile
  * reading every trace of its selection box, every trace is read for the whole
  * output grid once.  The panel is cut into segments of segment_traces traces
- * (0: 64 staged chunks; midpoint order, pstm_b200.spatial, keeps segments
+ * (0: 64 chunks of 32; midpoint order, pstm_b200.spatial, keeps segments
  * compact); on the device, each segment's midpoint box grown by the maximum
  * aperture is mapped to pillar blocks by binary search in the ascending grid
- * axes, the item counts are prefix-summed, and one persistent launch
- * migrates (segment, pillar block, time block) items with FP32 partial sums
- * per chunk and one atomic add per output sample per item.  Same result as
+ * axes, and one launch migrates the (segment, pillar block, time block) items:
+ * every CTA walks the segments that reach its block and adds into the image once.  Same result as
  * pstm_cuda_migrate_tile_dev up to the order of floating-point additions;
  * regular grids (x_axis, y_axis) and linear interpolation only.  Device
  * pointers; asynchronous on `stream`, except that a non-null n_items_out
@@ -205,16 +202,15 @@ int32_t pstm_cuda_migrate_tile_host(void *ctx, const pstm_traces_desc *traces,
  * device memory while they run -- an application whose memory manager owns
  * the whole GPU, or a job that must not stall the device (cudaMalloc
  * synchronises it) or fail on an allocation after start-up.  It needs no
- * context and allocates nothing: its scratch (tables, packed geometry, launch
- * parameters) is a fixed 16 MiB array in this library's device memory, held
- * by every device that loads the library until the process exits.  Limits of
+ * context and allocates nothing: launch parameters travel with the launch, and
+ * the kernel's error word is a variable of this library.  Limits of
  * one call: n_traces <= 131072, nt <= 8192, and (nx*ny if the velocity or eta
  * is 3-D, else 1) * nt <= 262144; larger inputs are rejected with
  * PSTM_ERR_INVALID_ARGUMENT (split the traces over several calls: image and
  * fold accumulate).  Inputs and outputs are device pointers; work is queued
  * on `stream` (NULL = the legacy default stream) of the calling thread's
- * current device.  The first call on a device looks up the array's address;
- * make that first call before any stream capture.  All calls share the array,
+ * current device.  The first call on a device looks up the word's address;
+ * make that first call before any stream capture.  All calls share the word,
  * so calls that overlap on the GPU race: serialise them.  The call is
  * asynchronous: its return status covers argument checks and launches, and
  * device-side failures are read afterwards with pstm_cuda_noalloc_status.
@@ -226,7 +222,7 @@ int32_t pstm_cuda_migrate_tile_noalloc(const pstm_traces_desc *traces, const pst
 /* Device-side status of the last pstm_cuda_migrate_tile_noalloc call on the
  * current device (no reference counterpart; the allocation-free form has
  * none).  Waits for `stream` (NULL = the legacy default stream), then reads the
- * kernel's error word from the fixed scratch array without allocating:
+ * kernel's error word without allocating:
  * PSTM_OK, or PSTM_ERR_TIMEOUT when a bounded device-side wait gave up -- the
  * image and fold of that call may then hold partial sums and must be
  * discarded.  Each allocation-free call clears the word when it starts. */
@@ -259,7 +255,7 @@ typedef struct {
 /* Launch shape chosen by pstm_cuda_autotune_bins. */
 typedef struct {
     int32_t pillars_per_cta;      /* output traces one CTA migrates together */
-    int32_t times_per_lane;       /* output times per thread (512 * this per CTA) */
+    int32_t times_per_lane;       /* output times per thread (32 * this per CTA) */
     int32_t traces_per_chunk;     /* depth of the staged trace panel */
     int32_t n_candidates;         /* shapes timed */
     float best_ms;                /* time of the chosen shape on the tuning sample */
@@ -267,15 +263,14 @@ typedef struct {
 } pstm_tune_result;
 
 /* Migrate many bins that share one output tile geometry, velocity and
- * parameters in ONE persistent launch: one CTA per SM takes (bin, pillar
- * block, time block) items from a work counter, the bins with the most traces
- * first, so bins of very different sizes keep every SM busy.  The whole
- * sequence (table preparation, geometry packing, the launch) is captured in a
- * CUDA graph that the context keeps and replays while the arguments repeat;
+ * parameters in ONE launch whose CTAs are (bin, time block, pillar block), the
+ * bins with the most traces first, so bins of very different sizes keep every
+ * SM busy.  The whole sequence (work list, the launch) is captured in a CUDA
+ * graph that the context keeps and replays while the arguments repeat;
  * new arguments re-capture it.  `output` gives the tile geometry (its image
  * and fold pointers are ignored; each bin has its own, and they must not
  * overlap).  Device pointers; asynchronous on `stream` as
- * pstm_cuda_migrate_tile_dev; at most 4096 bins.  Uses the shape that
+ * pstm_cuda_migrate_tile_dev; at most 4096 bins.  Uses the depth that
  * pstm_cuda_autotune_bins chose for this class of workload, if it ran.
  * Replaces the per-bin sequence of migrate_tile calls of the executor
  * (executor.py:960-975 -> :1730). */
@@ -286,8 +281,7 @@ int32_t pstm_cuda_migrate_bins_dev(void *ctx, const pstm_traces_desc *traces, co
 /* Autotuner of the batched form (no reference counterpart; the reference
  * picks its threadgroup shape by a fixed rule, compute_optimal_threadgroup,
  * pstm/kernels/metal_compiled.py:292-335, used at :742-743).  Times
- * candidate launch shapes (pillars per CTA, output times per lane, traces per
- * chunk) on a sample of the batch -- the largest bins, clipped so that one
+ * candidate depths (traces per chunk) on a sample of the batch -- the largest bins, clipped so that one
  * candidate migrates about `pairs_per_candidate` sample-trace pairs (0: 2^36)
  * into scratch outputs of the context -- keeps the fastest for this class of
  * workload (traveltime kind, trace dtype, 3-D velocity, precision, nt, ns) and

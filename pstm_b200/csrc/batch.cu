@@ -4,10 +4,9 @@
 //
 // The reference migrates its gather bins one after another, each bin a
 // sequence of per-tile kernel calls (pstm/pipeline/executor.py:960-975).
-// Here the bins of a tile are one launch: one CTA per SM takes items (bin,
-// pillar block, time block) from a work counter; the bins are ordered by
-// decreasing trace count, so the long items start first and bins of very
-// different sizes still end together.
+// Here the bins of a tile are one launch whose CTAs are (bin, time block,
+// pillar block); the bins are ordered by decreasing trace count, so the long
+// items start first and bins of very different sizes still end together.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdio>
@@ -30,13 +29,22 @@ namespace {
 
 constexpr int kMaxBins = 4096;
 
+// Work descriptors carried by value into store_bins (kernel parameters are
+// limited to 4 KB), so that they need no staging buffer and can be captured.
+constexpr int kBinsPerStore = 64;
+struct BinStore {
+    int32_t first, count;
+    BinWork w[kBinsPerStore];
+};
+__global__ void store_bins(const BinStore b, BinWork *dst) {
+    for (int i = threadIdx.x; i < b.count; i += blockDim.x) dst[b.first + i] = b.w[i];
+}
+
 struct BatchPlan {
     KParams P;
     Launch L;
     int tt = 0, amp = 0;
-    bool per_pillar = false, exact = false;
     int prec = PSTM_PREC_EXACT;   // pstm_precision
-    int64_t n_p = 0;
     std::vector<BinWork> work;   // non-empty bins, most traces first
 };
 
@@ -89,7 +97,7 @@ int32_t check_bins(Ctx *c, const pstm_traces_desc *tr, const pstm_output_desc *o
 // makes sure every buffer exists and fills the plan.  Allocates; enqueues
 // nothing.  bp.work is empty when there is nothing to migrate.
 int32_t plan_batch(Ctx *c, const pstm_traces_desc *tr, const pstm_output_desc *out, const pstm_velocity_desc *vel,
-                   const pstm_params *prm, const pstm_bin_desc *bins, int32_t n_bins, const Shape *force,
+                   const pstm_params *prm, const pstm_bin_desc *bins, int32_t n_bins, int force_chunk,
                    BatchPlan &bp) {
     int32_t rc = check_bins(c, tr, out, bins, n_bins);
     if (rc) return rc;
@@ -109,123 +117,44 @@ int32_t plan_batch(Ctx *c, const pstm_traces_desc *tr, const pstm_output_desc *o
     std::stable_sort(bp.work.begin(), bp.work.end(),
                      [](const BinWork &a, const BinWork &b) { return a.n_traces > b.n_traces; });
 
-    int R, PB, chunk = 0;
-    if (force) {
-        R = force->r;
-        PB = force->pb;
-        chunk = force->chunk;
-    } else {
-        plan::choose_shape(out->nt, c->force_r, c->force_pb, R, PB, tr->amp_dtype);
-        auto it = c->tuned.find(class_key(tr, out, vel, prm));
-        if (it != c->tuned.end() && !c->force_r && !c->force_pb) {
-            R = it->second.r;
-            PB = it->second.pb;
-            chunk = it->second.chunk;
-        }
-    }
-    if (R < 1 || R > 8 || PB < 1 || PB > kMaxPB) return fail(c, PSTM_ERR_INVALID_ARGUMENT, "launch shape out of range");
-
+    if (!plan::row_fits(tr, prm, out->nt, c->smem_optin))
+        return fail(c, PSTM_ERR_UNSUPPORTED, "trace rows too long to stage in shared memory");
     KParams &P = bp.P;
-    P = plan::make_params(tr, &o, vel, prm, PB);
+    P = plan::make_params(tr, &o, vel, prm);
+    if (force_chunk > 0) {
+        P.max_chunk = force_chunk;
+    } else {
+        auto it = c->tuned.find(class_key(tr, out, vel, prm));
+        if (it != c->tuned.end()) P.max_chunk = it->second;
+    }
     bp.tt = prm->traveltime;
     bp.amp = tr->amp_dtype;
-    bp.per_pillar = vel->is_3d || (prm->eta && prm->eta_is_3d);
-    bp.exact = prm->precision == PSTM_PREC_EXACT;
     bp.prec = prm->precision;
-    P.exact_units = bp.exact ? 1 : 0;
-    P.curved_kind = (prm->traveltime == PSTM_TT_CURVED || prm->traveltime == PSTM_TT_CURVED_VTI) ? 1 : 0;
-    bp.n_p = bp.per_pillar ? (int64_t)out->nx * out->ny : 1;
-    const size_t n_tab = (size_t)bp.n_p * out->nt;
     cudaError_t e;
-    if ((e = ensure(c->ttab, n_tab * sizeof(float4))) != cudaSuccess ||
-        (e = ensure(c->btab, n_tab * sizeof(double))) != cudaSuccess ||
-        (e = ensure(c->ttime, (size_t)out->nt * 2 * sizeof(float4))) != cudaSuccess ||
-        (e = ensure(c->ttimeA, (size_t)out->nt * sizeof(double))) != cudaSuccess ||
-        (e = ensure(c->ttimeV, (size_t)out->nt * sizeof(double))) != cudaSuccess ||
-        (e = ensure(c->errword, sizeof(int32_t))) != cudaSuccess ||
-        (e = ensure(c->kparams, sizeof(KParams))) != cudaSuccess ||
-        (e = ensure(c->packed_geo, (size_t)tr->n_traces * kGeoDoubles * sizeof(double))) != cudaSuccess ||
-        (e = ensure(c->bins, bp.work.size() * sizeof(BinWork))) != cudaSuccess ||
-        (e = ensure(c->counter, sizeof(unsigned long long))) != cudaSuccess)
+    if ((e = ensure(c->errword, sizeof(int32_t))) != cudaSuccess ||
+        (e = ensure(c->bins, bp.work.size() * sizeof(BinWork))) != cudaSuccess)
         return cuda_fail(c, e, "allocating the batch buffers");
-    P.ttab = reinterpret_cast<const float4 *>(c->ttab.ptr);
-    P.btab = reinterpret_cast<const double *>(c->btab.ptr);
-    P.ttime = reinterpret_cast<const float4 *>(c->ttime.ptr);
-    P.ttimeA = reinterpret_cast<const double *>(c->ttimeA.ptr);
-    P.ttimeV = reinterpret_cast<const double *>(c->ttimeV.ptr);
-    P.geo = reinterpret_cast<const double *>(c->packed_geo.ptr);
     P.err = reinterpret_cast<int32_t *>(c->errword.ptr);
-    size_t smem = 0;
-    if (!plan::plan_staging(P, tr, prm, PB, R, c->smem_optin, smem, chunk))
-        return fail(c, PSTM_ERR_UNSUPPORTED, "trace rows too long to stage in shared memory");
-
-    // bins much larger than L2 are split into trace segments (consecutive in the
-    // work list, so the resident CTAs share each segment in L2); split bins add
-    // into their outputs atomically
-    const int64_t row_bytes = (int64_t)P.pitch * P.elem;
-    if (c->segment_bytes > 0) {
-        int64_t S = c->segment_bytes / row_bytes;
-        S = S < 16 * (int64_t)P.chunk ? 16 * (int64_t)P.chunk : S / P.chunk * P.chunk;
-        std::vector<BinWork> split;
-        for (const BinWork &w : bp.work) {
-            if (w.n_traces * row_bytes <= 2 * c->segment_bytes) {
-                split.push_back(w);
-                continue;
-            }
-            for (int64_t b = 0; b < w.n_traces; b += S)
-                split.push_back({w.trace0 + b, (w.n_traces - b) < S ? (w.n_traces - b) : S, w.image, w.fold});
-            P.atomic_flush = 1;
-        }
-        if (split.size() > (size_t)(64 * kMaxBins))
-            return fail(c, PSTM_ERR_UNSUPPORTED, "too many trace segments in one batch");
-        bp.work.swap(split);
-        if ((e = ensure(c->bins, bp.work.size() * sizeof(BinWork))) != cudaSuccess)
-            return cuda_fail(c, e, "allocating the batch work list");
-    }
-
+    P.bins = reinterpret_cast<const BinWork *>(c->bins.ptr);
+    P.n_bins = (int32_t)bp.work.size();
     bp.L = Launch();
-    bp.L.smem = smem;
-    bp.L.bins = reinterpret_cast<const BinWork *>(c->bins.ptr);
-    bp.L.n_bins = (int)bp.work.size();
-    bp.L.counter = reinterpret_cast<unsigned long long *>(c->counter.ptr);
-    // resolve the CTA count and the shared-memory opt-in now: nothing but
-    // stream work may happen while the launch sequence is captured
-    unsigned ctas = 0;
+    if (!plan::plan_grid(P, P.n_bins, bp.L.grid)) return fail(c, PSTM_ERR_UNSUPPORTED, "batch too large for one launch");
+    bp.L.smem = plan::gather_smem(prm->traveltime);
+    // resolve the shared-memory opt-in now: nothing but stream work may happen
+    // while the launch sequence is captured
     bp.L.configure_only = true;
-    bp.L.ctas_out = &ctas;
-    e = launch_kind(bp.tt, P, reinterpret_cast<const KParams *>(c->kparams.ptr), bp.amp, bp.per_pillar, bp.prec,
-                    bp.L);
-    if (e != cudaSuccess) return cuda_fail(c, e, "configuring the persistent kernel");
+    e = launch_kind(bp.tt, P, bp.prec, bp.L);
+    if (e != cudaSuccess) return cuda_fail(c, e, "configuring the gather kernel");
     bp.L.configure_only = false;
-    bp.L.ctas_out = nullptr;
-    bp.L.grid = dim3(ctas);
     return PSTM_OK;
 }
 
-// Enqueues the whole batch on `st`: error word and work counter cleared,
-// tables, packed geometry, parameter block, work list, the persistent launch.
+// Enqueues the whole batch on `st`: error word cleared, work list, the launch.
 // Allocates nothing, so it can be captured.
 int32_t enqueue_batch(Ctx *c, BatchPlan &bp, cudaStream_t st) {
-    KParams &P = bp.P;
     cudaError_t e;
-    if ((e = cudaMemsetAsync(c->errword.ptr, 0, sizeof(int32_t), st)) != cudaSuccess ||
-        (e = cudaMemsetAsync(c->counter.ptr, 0, sizeof(unsigned long long), st)) != cudaSuccess)
-        return cuda_fail(c, e, "clearing the error word and work counter");
-    const int64_t n_tab = bp.n_p * P.nt;
-    int blocks = (int)std::min<int64_t>((n_tab + 255) / 256, 148 * 32);
-    prep_time_table<<<blocks, 256, 0, st>>>(P, bp.n_p, reinterpret_cast<float4 *>(c->ttab.ptr),
-                                            reinterpret_cast<double *>(c->btab.ptr),
-                                            reinterpret_cast<float4 *>(c->ttime.ptr),
-                                            reinterpret_cast<double *>(c->ttimeA.ptr),
-                                            reinterpret_cast<double *>(c->ttimeV.ptr));
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "prep_time_table launch");
-    blocks = (int)std::min<int64_t>((P.n_traces + 255) / 256, 148 * 32);
-    if (blocks > 0) {
-        pack_geometry<<<blocks, 256, 0, st>>>(P, reinterpret_cast<double *>(c->packed_geo.ptr));
-        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "pack_geometry launch");
-    }
-    store_params<<<1, 32, 0, st>>>(P, reinterpret_cast<KParams *>(c->kparams.ptr));
-    if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "store_params launch");
+    if ((e = cudaMemsetAsync(c->errword.ptr, 0, sizeof(int32_t), st)) != cudaSuccess)
+        return cuda_fail(c, e, "clearing the error word");
     for (size_t i = 0; i < bp.work.size(); i += kBinsPerStore) {
         BinStore b;
         std::memset(&b, 0, sizeof(b));
@@ -236,9 +165,8 @@ int32_t enqueue_batch(Ctx *c, BatchPlan &bp, cudaStream_t st) {
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "store_bins launch");
     }
     bp.L.stream = st;
-    e = launch_kind(bp.tt, P, reinterpret_cast<const KParams *>(c->kparams.ptr), bp.amp, bp.per_pillar, bp.prec,
-                    bp.L);
-    if (e != cudaSuccess) return cuda_fail(c, e, "persistent migrate kernel launch");
+    e = launch_kind(bp.tt, bp.P, bp.prec, bp.L);
+    if (e != cudaSuccess) return cuda_fail(c, e, "batched migrate kernel launch");
     return PSTM_OK;
 }
 
@@ -252,8 +180,7 @@ std::vector<unsigned char> graph_key(const BatchPlan &bp) {
     };
     put(&bp.P, sizeof(KParams));
     if (!bp.work.empty()) put(bp.work.data(), bp.work.size() * sizeof(BinWork));
-    const int64_t extra[8] = {bp.tt, bp.amp, bp.per_pillar, bp.prec, (int64_t)bp.L.grid.x, (int64_t)bp.L.smem,
-                              (int64_t)(uintptr_t)bp.L.bins, (int64_t)(uintptr_t)bp.L.counter};
+    const int64_t extra[5] = {bp.tt, bp.amp, bp.prec, (int64_t)bp.L.grid, (int64_t)bp.L.smem};
     put(extra, sizeof(extra));
     return k;
 }
@@ -307,12 +234,9 @@ void release_batch(Ctx *c) {
     c->graph = nullptr;
     c->graph_key.clear();
     release(c->bins);
-    release(c->counter);
     release(c->tune_image);
     release(c->tune_fold);
     release(c->probe);
-    release(c->seg_bins);
-    release(c->seg_counter);
 }
 }  // namespace ctx
 }  // namespace pstm
@@ -329,7 +253,7 @@ int32_t pstm_cuda_migrate_bins_dev(void *ctx, const pstm_traces_desc *traces, co
     cudaError_t e = cudaSetDevice(c->device);
     if (e != cudaSuccess) return cuda_fail(c, e, "cudaSetDevice");
     BatchPlan bp;
-    int32_t rc = plan_batch(c, traces, output, velocity, params, bins, n_bins, nullptr, bp);
+    int32_t rc = plan_batch(c, traces, output, velocity, params, bins, n_bins, 0, bp);
     if (rc || bp.work.empty()) return rc;
     cudaStream_t st = stream ? reinterpret_cast<cudaStream_t>(stream) : c->stream;
     return graphs_enabled() ? run_graph(c, bp, st) : enqueue_batch(c, bp, st);
@@ -378,37 +302,21 @@ int32_t pstm_cuda_autotune_bins(void *ctx, const pstm_traces_desc *traces, const
         big[i].fold = reinterpret_cast<int32_t *>(static_cast<unsigned char *>(c->tune_fold.ptr) + i * fold_bytes);
     }
 
-    // candidates: the default shape first, then pillars per CTA x times per
-    // lane x panel depth
-    Shape def;
-    plan::choose_shape(o.nt, 0, 0, def.r, def.pb, traces->amp_dtype);
-    std::vector<Shape> cand{def};
-    std::vector<int> rs{def.r};
-    if (def.r > 1) rs.push_back((def.r + 1) / 2);
-    for (int r : rs)
-        for (int pb : {2, 4, 8})
-            for (int ch : {0, 16, 8}) {
-                Shape s{pb, r, ch};
-                if (!(s.pb == def.pb && s.r == def.r && s.chunk == 0)) cand.push_back(s);
-            }
+    // candidates: traces staged per step, the default (as many as fit) first
+    const int cand[] = {kChunk, kChunk * 3 / 4, kChunk / 2, kChunk / 4};
 
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     if ((e = cudaEventCreate(&ev0)) != cudaSuccess || (e = cudaEventCreate(&ev1)) != cudaSuccess) {
         if (ev0) cudaEventDestroy(ev0);
         return cuda_fail(c, e, "cudaEventCreate");
     }
-    Shape best = def;
+    int best = kChunk;
     float best_ms = -1.f, default_ms = -1.f;
     int timed = 0;
-    for (const Shape &s : cand) {
+    for (const int chunk : cand) {
         BatchPlan bp;
-        rc = plan_batch(c, traces, &o, velocity, params, big.data(), (int32_t)big.size(), &s, bp);
-        if (rc == PSTM_ERR_UNSUPPORTED) {   // does not fit in shared memory
-            rc = PSTM_OK;
-            continue;
-        }
+        rc = plan_batch(c, traces, &o, velocity, params, big.data(), (int32_t)big.size(), chunk, bp);
         if (rc) break;
-        if (s.chunk && bp.P.chunk != s.chunk) continue;   // deeper than fits: the same as chunk 0
         float ms = 1e30f;
         for (int rep = 0; rep < 2 && rc == PSTM_OK; ++rep) {   // the first run warms up
             if ((e = cudaEventRecord(ev0, c->stream)) != cudaSuccess) {
@@ -436,20 +344,19 @@ int32_t pstm_cuda_autotune_bins(void *ctx, const pstm_traces_desc *traces, const
             break;
         }
         ++timed;
-        const Shape eff{s.pb, s.r, s.chunk ? bp.P.chunk : 0};
         if (timed == 1) default_ms = ms;
         if (best_ms < 0.f || ms < best_ms) {
             best_ms = ms;
-            best = eff;
+            best = chunk;
         }
     }
     cudaEventDestroy(ev0);
     cudaEventDestroy(ev1);
     if (rc) return rc;
     c->tuned[class_key(traces, output, velocity, params)] = best;
-    result->pillars_per_cta = best.pb;
-    result->times_per_lane = best.r;
-    result->traces_per_chunk = best.chunk;
+    result->pillars_per_cta = kPillars;
+    result->times_per_lane = kTimes / 32;
+    result->traces_per_chunk = best;
     result->n_candidates = timed;
     result->best_ms = best_ms;
     result->default_ms = default_ms;

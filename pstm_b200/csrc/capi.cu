@@ -93,145 +93,30 @@ int32_t prepare_tile(Ctx *c, const pstm_traces_desc *tr, const pstm_output_desc 
     if (injected("migrate")) return fail(c, PSTM_ERR_INJECTED, "injected fault: migrate");
     cudaError_t e = cudaSetDevice(c->device);
     if (e != cudaSuccess) return cuda_fail(c, e, "cudaSetDevice");
-    int R, PB;
-    plan::choose_shape(out->nt, c->force_r, c->force_pb, R, PB, tr->amp_dtype);
     KParams &P = tp.P;
-    P = make_params(tr, out, vel, prm, PB);
+    P = make_params(tr, out, vel, prm);
     if (tr->n_traces == 0) return PSTM_OK;   // nothing to add: image += 0, fold += 0
-
-    const bool per_pillar = vel->is_3d || (prm->eta && prm->eta_is_3d);
-    const int64_t n_p = per_pillar ? (int64_t)out->nx * out->ny : 1;
-    const size_t n_tab = (size_t)n_p * out->nt;
-    if ((e = ensure(c->ttab, n_tab * sizeof(float4))) != cudaSuccess ||
-        (e = ensure(c->btab, n_tab * sizeof(double))) != cudaSuccess ||
-        (e = ensure(c->ttime, (size_t)out->nt * 2 * sizeof(float4))) != cudaSuccess ||
-        (e = ensure(c->ttimeA, (size_t)out->nt * sizeof(double))) != cudaSuccess ||
-        (e = ensure(c->ttimeV, (size_t)out->nt * sizeof(double))) != cudaSuccess ||
-        (e = ensure(c->errword, sizeof(int32_t))) != cudaSuccess)
-        return cuda_fail(c, e, "allocating the per-time tables");
-    float4 *tab = reinterpret_cast<float4 *>(c->ttab.ptr);
-    double *btab = reinterpret_cast<double *>(c->btab.ptr);
-    const bool exact = prm->precision == PSTM_PREC_EXACT;
-    P.exact_units = exact ? 1 : 0;
-    P.curved_kind = (prm->traveltime == PSTM_TT_CURVED || prm->traveltime == PSTM_TT_CURVED_VTI) ? 1 : 0;
-    {
-        int blocks = (int)(((int64_t)n_tab + 255) / 256);
-        if (blocks > 148 * 32) blocks = 148 * 32;
-        prep_time_table<<<blocks, 256, 0, st>>>(P, n_p, tab, btab, reinterpret_cast<float4 *>(c->ttime.ptr),
-                                                reinterpret_cast<double *>(c->ttimeA.ptr),
-                                                reinterpret_cast<double *>(c->ttimeV.ptr));
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return cuda_fail(c, e, "prep_time_table launch");
-    }
-    P.ttime = reinterpret_cast<const float4 *>(c->ttime.ptr);
-    P.ttimeA = reinterpret_cast<const double *>(c->ttimeA.ptr);
-    P.ttimeV = reinterpret_cast<const double *>(c->ttimeV.ptr);
-    P.ttab = tab;
-    P.btab = btab;
+    if (!plan::row_fits(tr, prm, out->nt, c->smem_optin))
+        return fail(c, PSTM_ERR_UNSUPPORTED, "trace rows too long to stage in shared memory");
+    if ((e = ensure(c->errword, sizeof(int32_t))) != cudaSuccess)
+        return cuda_fail(c, e, "allocating the error word");
     P.err = reinterpret_cast<int32_t *>(c->errword.ptr);
     if ((e = cudaMemsetAsync(P.err, 0, sizeof(int32_t), st)) != cudaSuccess)
         return cuda_fail(c, e, "clearing the error word");
-
-    // packed FP64 geometry, staged per chunk by TMA bulk copies
-    if ((e = ensure(c->packed_geo, (size_t)tr->n_traces * kGeoDoubles * sizeof(double))) != cudaSuccess)
-        return cuda_fail(c, e, "allocating the packed geometry");
-    {
-        int blocks = (int)((tr->n_traces + 255) / 256);
-        if (blocks > 148 * 32) blocks = 148 * 32;
-        pack_geometry<<<blocks, 256, 0, st>>>(P, reinterpret_cast<double *>(c->packed_geo.ptr));
-        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "pack_geometry launch");
-    }
-    P.geo = reinterpret_cast<const double *>(c->packed_geo.ptr);
-
-    // shared-memory staging of trace rows: pitch rounded up to 16 bytes; TMA
-    // bulk copies when the rows are 16-byte aligned and the padded row is
-    // inside the caller's stride, else a plain cooperative copy
-    size_t smem = 0;
-    if (!plan::plan_staging(P, tr, prm, PB, R, c->smem_optin, smem))
-        return fail(c, PSTM_ERR_UNSUPPORTED, "trace rows too long to stage in shared memory");
-
-    // a device copy of the launch parameters for the kernel's rare FP64 paths
-    e = ensure(c->kparams, sizeof(KParams));
-    if (e != cudaSuccess) return cuda_fail(c, e, "allocating the parameter block");
-    e = cudaMemcpyAsync(c->kparams.ptr, &P, sizeof(KParams), cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return cuda_fail(c, e, "copying the parameter block");
-    const KParams *Pg = reinterpret_cast<const KParams *>(c->kparams.ptr);
-
-    const int n_pblk_x = (out->nx + P.px - 1) / P.px;
-    const int64_t nblk_p = (int64_t)n_pblk_x * P.n_pblk_y;
-    const int tb = kThreads * R;
-    const int nblk_t = (out->nt + tb - 1) / tb;
-    if (nblk_p > 0x7fffffff || nblk_t > 65535) return fail(c, PSTM_ERR_UNSUPPORTED, "tile too large for one launch");
-    tp.Pg = Pg;
     tp.L = Launch();
-    tp.L.grid = dim3((unsigned)nblk_p, (unsigned)nblk_t);
-    tp.L.smem = smem;
+    if (!plan::plan_grid(P, 1, tp.L.grid)) return fail(c, PSTM_ERR_UNSUPPORTED, "tile too large for one launch");
+    tp.L.smem = plan::gather_smem(prm->traveltime);
     tp.L.stream = st;
     tp.tt = prm->traveltime;
     tp.amp = tr->amp_dtype;
-    tp.per_pillar = per_pillar;
-    tp.exact = exact;
+    tp.exact = prm->precision == PSTM_PREC_EXACT;
     tp.prec = prm->precision;
-    tp.n_p = n_p;
     tp.empty = false;
     return PSTM_OK;
 }
 
-// Trace-segment length of the segment-major schedule for this tile (0: the
-// context never splits).
-int64_t segment_traces(const Ctx *c, const KParams &P) {
-    if (c->segment_bytes <= 0) return 0;
-    const int64_t row_bytes = (int64_t)P.pitch * P.elem;
-    const int64_t S = c->segment_bytes / row_bytes;
-    return S < 16 * (int64_t)P.chunk ? 16 * (int64_t)P.chunk : S / P.chunk * P.chunk;
-}
-
-// Items for traces [b0, b0 + n) of the prepared panel, S traces at most each
-// (S <= 0: one item).
-void append_segments(std::vector<BinWork> &w, int64_t b0, int64_t n, int64_t S, void *image, int32_t *fold) {
-    if (S <= 0) S = n;
-    for (int64_t b = 0; b < n; b += S) w.push_back({b0 + b, (n - b) < S ? (n - b) : S, image, fold});
-}
-
-// One persistent launch over a list of trace items of the prepared tile, all
-// adding into its image and fold atomically.
-int32_t launch_items(Ctx *c, const TilePlan &tp, const std::vector<BinWork> &w) {
-    if (w.size() > (size_t)0x7fffffff) return fail(c, PSTM_ERR_UNSUPPORTED, "too many trace items for one launch");
-    cudaError_t e;
-    if ((e = ensure(c->seg_bins, w.size() * sizeof(BinWork))) != cudaSuccess ||
-        (e = ensure(c->seg_counter, sizeof(unsigned long long))) != cudaSuccess)
-        return cuda_fail(c, e, "allocating the segment list");
-    if ((e = cudaMemcpyAsync(c->seg_bins.ptr, w.data(), w.size() * sizeof(BinWork), cudaMemcpyHostToDevice,
-                             tp.L.stream)) != cudaSuccess ||
-        (e = cudaMemsetAsync(c->seg_counter.ptr, 0, sizeof(unsigned long long), tp.L.stream)) != cudaSuccess)
-        return cuda_fail(c, e, "writing the segment list");
-    KParams P = tp.P;
-    P.atomic_flush = 1;
-    Launch L;
-    L.smem = tp.L.smem;
-    L.stream = tp.L.stream;
-    L.bins = reinterpret_cast<const BinWork *>(c->seg_bins.ptr);
-    L.n_bins = (int)w.size();
-    L.counter = reinterpret_cast<unsigned long long *>(c->seg_counter.ptr);
-    e = launch_kind(tp.tt, P, tp.Pg, tp.amp, tp.per_pillar, tp.prec, L);
-    return e == cudaSuccess ? PSTM_OK : cuda_fail(c, e, "segmented migrate kernel launch");
-}
-
-// A panel much larger than L2 is migrated segment by segment: the persistent
-// kernel takes items (trace segment, pillar block, time block) in segment
-// order, so every resident CTA streams the same L2-sized segment at a time
-// and the panel is read from DRAM about once instead of once per CTA; the
-// items of a pillar block in different segments add into the image and fold
-// atomically.
 int32_t launch_tile(Ctx *c, const TilePlan &tp) {
-    const KParams &P0 = tp.P;
-    const int64_t row_bytes = (int64_t)P0.pitch * P0.elem;
-    if (c->segment_bytes > 0 && P0.n_traces * row_bytes > 2 * c->segment_bytes) {
-        std::vector<BinWork> w;
-        append_segments(w, 0, P0.n_traces, segment_traces(c, P0), P0.image, P0.fold);
-        return launch_items(c, tp, w);
-    }
-    const cudaError_t e = launch_kind(tp.tt, tp.P, tp.Pg, tp.amp, tp.per_pillar, tp.prec, tp.L);
+    const cudaError_t e = launch_kind(tp.tt, tp.P, tp.prec, tp.L);
     return e == cudaSuccess ? PSTM_OK : cuda_fail(c, e, "migrate kernel launch");
 }
 
@@ -312,12 +197,6 @@ int32_t pstm_cuda_create(int32_t device, void **ctx_out) {
         delete c;
         return cuda_fail(nullptr, e, "cudaDeviceGetAttribute");
     }
-    const char *rr = std::getenv("PSTM_CUDA_R");   // output times per lane override (1..4)
-    if (rr) c->force_r = std::atoi(rr);
-    const char *pb = std::getenv("PSTM_CUDA_PB");   // pillars per CTA override (1..16)
-    if (pb) c->force_pb = std::atoi(pb);
-    const char *seg = std::getenv("PSTM_CUDA_SEGMENT_MB");   // trace-segment size; 0: never split a panel
-    if (seg) c->segment_bytes = (int64_t)std::atoll(seg) << 20;
     *ctx_out = c;
     return PSTM_OK;
 }
@@ -327,18 +206,13 @@ void pstm_cuda_destroy(void *ctx) {
     if (!c) return;
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
-    release(c->ttab);
-    release(c->btab);
-    release(c->ttime);
-    release(c->ttimeA);
-    release(c->ttimeV);
-    release(c->kparams);
     release(c->errword);
-    release(c->packed_geo);
     release(c->amps);
     for (auto &g : c->geo) release(g);
     release(c->xa); release(c->ya); release(c->xg); release(c->yg); release(c->ta);
     release(c->vel); release(c->eta); release(c->image); release(c->fold);
+    release(c->runs);
+    release(c->seg_boxes);
     release(c->scatter_ends);
     release_batch(c);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -402,16 +276,24 @@ int32_t pstm_cuda_migrate_tile_runs_dev(void *ctx, const pstm_traces_desc *trace
         }
         return PSTM_OK;
     }
-    // One tile preparation over the span of the runs (geometry packed for the
-    // span) and one persistent launch over the runs' segments.
-    const int64_t a0 = rv.front().first;
-    const pstm_traces_desc span = sub_panel(*traces, a0, rv.back().second - a0);
+    // One launch whose CTAs walk the ranges.
     TilePlan tp;
-    if ((rc = prepare_tile(c, &span, output, velocity, params, st, tp)) != PSTM_OK || tp.empty) return rc;
-    const int64_t S = segment_traces(c, tp.P);
-    std::vector<BinWork> w;
-    for (const auto &r : rv) append_segments(w, r.first - a0, r.second - r.first, S, tp.P.image, tp.P.fold);
-    return launch_items(c, tp, w);
+    if ((rc = prepare_tile(c, traces, output, velocity, params, st, tp)) != PSTM_OK || tp.empty) return rc;
+    cudaError_t e;
+    if ((e = ensure(c->runs, rv.size() * 2 * sizeof(int64_t))) != cudaSuccess)
+        return cuda_fail(c, e, "allocating the run list");
+    std::vector<int64_t> flat;
+    for (const auto &r : rv) {
+        flat.push_back(r.first);
+        flat.push_back(r.second);
+        tp.P.n_run_traces += r.second - r.first;
+    }
+    if ((e = cudaMemcpyAsync(c->runs.ptr, flat.data(), flat.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st)) !=
+        cudaSuccess)
+        return cuda_fail(c, e, "writing the run list");
+    tp.P.runs = reinterpret_cast<const int64_t *>(c->runs.ptr);
+    tp.P.n_runs = (int32_t)rv.size();
+    return launch_tile(c, tp);
 }
 
 static int32_t migrate_host_impl(Ctx *c, const pstm_traces_desc *traces, const pstm_output_desc *output,

@@ -1,6 +1,6 @@
 // ctx.h -- the context behind a pstm_cuda handle: its stream, the device
 // buffers it reuses from call to call, and the state of the batched form
-// (cached CUDA graph, tuned launch shapes).
+// (cached CUDA graph, tuned chunk depths).
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -19,43 +19,32 @@ struct DevBuf {
     size_t bytes = 0;
 };
 
-// Launch shape of the gather kernels: pillars per CTA, output times per lane,
-// traces per staged chunk (0: as many as shared memory holds).
-struct Shape {
-    int pb = 0, r = 0, chunk = 0;
-};
-
 struct Ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
     std::string err;
-    DevBuf ttab, btab, ttime, ttimeA, ttimeV, kparams, errword, packed_geo;
+    DevBuf errword;
     // staging for the host-pointer path
     DevBuf amps, geo[7], xa, ya, xg, yg, ta, vel, eta, image, fold;
-    int force_r = 0;      // PSTM_CUDA_R override of the output times per lane
-    int force_pb = 0;     // PSTM_CUDA_PB override of the pillars per CTA
     int smem_optin = 0;   // max dynamic shared memory per block
     // batched form
-    DevBuf bins, counter, tune_image, tune_fold;
+    DevBuf bins, tune_image, tune_fold;
     DevBuf probe;                           // learned form: per-probe residuals
-    DevBuf seg_bins, seg_counter;           // per-tile launches split into trace segments
-    DevBuf scatter_ends;                    // scatter schedule: prefix counts of the segments' items
-    int64_t segment_bytes = 24ll << 20;     // trace-panel bytes per segment (0: never split)
+    DevBuf runs;                            // trace ranges of a call on runs
+    DevBuf seg_boxes, scatter_ends;         // scatter schedule: the segments' boxes, prefix counts of their items
     std::vector<unsigned char> graph_key;   // arguments the cached graph was captured with
     cudaGraphExec_t graph = nullptr;
-    std::map<std::string, Shape> tuned;     // autotuned shapes by workload class
+    std::map<std::string, int> tuned;       // autotuned traces per chunk by workload class
 };
 
-// A per-tile launch prepared by prepare_tile: tables, packed geometry and the
-// device parameter block are enqueued; the migration launch is not.
+// A launch prepared by prepare_tile: the parameters and grid of one tile, its
+// error word cleared; the migration launch is not enqueued.
 struct TilePlan {
     KParams P;
-    const KParams *Pg = nullptr;
     Launch L;
     int tt = 0, amp = 0;
-    bool per_pillar = false, exact = false;
+    bool exact = false;
     int prec = PSTM_PREC_EXACT;   // pstm_precision of the launch
-    int64_t n_p = 0;
     bool empty = true;   // no traces: nothing to launch
 };
 

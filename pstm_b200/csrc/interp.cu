@@ -11,7 +11,7 @@
 // FP32 taps, interpolation and weights after the FP64 sample index on the fast
 // path -- with one CTA of 128
 // threads per (pillar, block of 128 output times) and the traces read from
-// the packed geometry and the caller's panel.  Each warp stages the traces 32
+// the caller's geometry and panel.  Each warp stages the traces 32
 // at a time in a shared-memory slice of its own: each lane takes one trace's
 // pillar distances, counts it for the fold and keeps it if it lies inside the
 // largest aperture of the warp's times; the kept traces, in trace order, go to
@@ -217,10 +217,9 @@ __global__ void __launch_bounds__(kInterpThreads, PSTM_INTERP_MIN_CTAS) migrate_
         const int64_t tr = c0 + lane;
         bool keep = false, in_fold = false;
         double dxm = 0.0, dym = 0.0, d = 0.0;
-        const double *g = P.geo + tr * kGeoDoubles;
         if (tr < P.n_traces) {
-            dxm = ox - g[4];
-            dym = oy - g[5];
+            dxm = ox - P.mx[tr];
+            dym = oy - P.my[tr];
             const double d2 = dxm * dxm + dym * dym;
             in_fold = d2 <= P.fold_d2_max;
             d = sqrt(d2);
@@ -231,11 +230,11 @@ __global__ void __launch_bounds__(kInterpThreads, PSTM_INTERP_MIN_CTAS) migrate_
         const int n_kept = __popc(kb);
         if (keep) {
             const int j = __popc(kb & ((1u << lane) - 1u));
-            const double dxs = ox - g[0], dys = oy - g[1], dxr = ox - g[2], dyr = oy - g[3];
+            const double dxs = ox - P.sx[tr], dys = oy - P.sy[tr], dxr = ox - P.rx[tr], dyr = oy - P.ry[tr];
             S.ds2[j] = dxs * dxs + dys * dys;
             S.dr2[j] = dxr * dxr + dyr * dyr;
             S.d[j] = d;
-            S.w[j] = g[6];
+            S.w[j] = P.w ? P.w[tr] : 1.0;
             S.m[j] = fmax(fabs(dxm), fabs(dym));
             S.tr[j] = (int)tr;
         }

@@ -33,64 +33,40 @@ static cudaError_t opt_in_smem(SmemOptIn &state, Kernel kern, size_t smem) {
     return e;
 }
 
-template <int TT, int AMP, bool VEL3D, bool EXACT, bool W2, bool GUARD>
-static cudaError_t launch_w(const KParams &P, const KParams *Pg, const Launch &L) {
-    if (!L.bins && !L.scatter.boxes) {
-        auto kern = migrate_kernel<TT, AMP, VEL3D, EXACT, W2, GUARD>;
-        static SmemOptIn opt_in;   // per instantiation
-        cudaError_t e = opt_in_smem(opt_in, kern, L.smem);
-        if (e != cudaSuccess) return e;
-        kern<<<L.grid, kThreads, L.smem, L.stream>>>(P, Pg);
-        return cudaGetLastError();
-    }
-    auto kern = migrate_persistent_kernel<TT, AMP, VEL3D, EXACT, W2, GUARD>;
-    static SmemOptIn opt_in;
-    {
-        cudaError_t e = opt_in_smem(opt_in, kern, L.smem);
-        if (e != cudaSuccess) return e;
-    }
-    unsigned ctas = L.grid.x;
-    if (ctas == 0) {
-        int dev = 0, sms = 0, per_sm = 0;
-        cudaError_t e = cudaGetDevice(&dev);
-        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, L.smem);
-        if (e != cudaSuccess) return e;
-        ctas = (unsigned)(sms * (per_sm > 0 ? per_sm : 1));
-    }
-    if (L.configure_only) {
-        if (L.ctas_out) *L.ctas_out = ctas;
-        return cudaSuccess;
-    }
-    kern<<<ctas, kThreads, L.smem, L.stream>>>(P, Pg, L.bins, L.n_bins, L.counter, L.scatter);
-    return cudaGetLastError();
+template <int TT, int PREC, bool W2, bool AA>
+static cudaError_t launch_one(const KParams &P, const Launch &L) {
+    auto kern = gather_kernel<TT, PREC, W2, AA>;
+    static SmemOptIn opt_in;   // per instantiation
+    cudaError_t e = opt_in_smem(opt_in, kern, L.smem);
+    if (e != cudaSuccess || L.configure_only) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(L.grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = L.smem;
+    cfg.stream = L.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)P.n_splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = P.n_splits > 1 ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, kern, P);
+    return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
-template <int TT, int AMP, bool VEL3D, bool EXACT, bool GUARD>
-static cudaError_t launch_one(const KParams &P, const KParams *Pg, const Launch &L) {
-    if (P.spreading && P.obliquity) return launch_w<TT, AMP, VEL3D, EXACT, true, GUARD>(P, Pg, L);
-    return launch_w<TT, AMP, VEL3D, EXACT, false, GUARD>(P, Pg, L);
+template <int TT, int PREC>
+static cudaError_t launch_prec(const KParams &P, const Launch &L) {
+    const bool w2 = P.spreading && P.obliquity;
+    if (P.aa) return w2 ? launch_one<TT, PREC, true, true>(P, L) : launch_one<TT, PREC, false, true>(P, L);
+    return w2 ? launch_one<TT, PREC, true, false>(P, L) : launch_one<TT, PREC, false, false>(P, L);
 }
 
-template <int TT, bool EXACT, bool GUARD>
-static cudaError_t launch_prec(const KParams &P, const KParams *Pg, int amp, bool vel3d, const Launch &L) {
-#define PSTM_CASE(A_, V_) \
-    if (amp == A_ && vel3d == V_) return launch_one<TT, A_, V_, EXACT, GUARD>(P, Pg, L);
-    PSTM_CASE(AMP_F32, false) PSTM_CASE(AMP_F32, true)
-    PSTM_CASE(AMP_BF16, false) PSTM_CASE(AMP_BF16, true)
-    PSTM_CASE(AMP_F16, false) PSTM_CASE(AMP_F16, true)
-#undef PSTM_CASE
-    return cudaErrorInvalidValue;
-}
-
-// prec: PSTM_PREC_EXACT the FP64 sample index; PSTM_PREC_FAST FP32 traveltime with
-// FP64 re-decisions of the trace-end tests in a guard band; PSTM_PREC_FP32 FP32
-// traveltime, sample index and trace-end tests (no guard band).
 template <int TT>
-cudaError_t launch_migrate(const KParams &P, const KParams *Pg, int amp, bool vel3d, int prec, const Launch &L) {
-    if (prec == PSTM_PREC_EXACT) return launch_prec<TT, true, true>(P, Pg, amp, vel3d, L);
-    if (prec == PSTM_PREC_FAST) return launch_prec<TT, false, true>(P, Pg, amp, vel3d, L);
-    return launch_prec<TT, false, false>(P, Pg, amp, vel3d, L);
+cudaError_t launch_gather(const KParams &P, int prec, const Launch &L) {
+    if (prec == PSTM_PREC_EXACT) return launch_prec<TT, PSTM_PREC_EXACT>(P, L);
+    if (prec == PSTM_PREC_FAST) return launch_prec<TT, PSTM_PREC_FAST>(P, L);
+    return launch_prec<TT, PSTM_PREC_FP32>(P, L);
 }
 
 }  // namespace pstm

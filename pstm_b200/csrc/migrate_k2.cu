@@ -1,5 +1,5 @@
 // Instantiations of the gather kernel for traveltime kind 2.
 #include "migrate_dispatch.cuh"
 namespace pstm {
-template cudaError_t launch_migrate<2>(const KParams &, const KParams *, int, bool, int, const Launch &);
+template cudaError_t launch_gather<2>(const KParams &, int, const Launch &);
 }

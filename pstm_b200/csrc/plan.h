@@ -1,6 +1,5 @@
 // plan.h -- host-side launch planning shared by the entry points: argument
-// checks, launch parameters, and the split of shared memory between staged
-// trace rows, records and partial sums.
+// checks, launch parameters and the grid.
 #pragma once
 #include <cuda_runtime.h>
 #include <cmath>
@@ -65,10 +64,14 @@ inline int32_t check_args(const pstm_traces_desc *tr, const pstm_output_desc *ou
 }
 
 inline KParams make_params(const pstm_traces_desc *tr, const pstm_output_desc *out, const pstm_velocity_desc *vel,
-                    const pstm_params *prm, int PB) {
+                    const pstm_params *prm) {
     KParams P;
     std::memset(&P, 0, sizeof(P));
     P.amps = tr->amplitudes;
+    P.amp_kind = tr->amp_dtype;
+    P.amps_end = static_cast<const unsigned char *>(tr->amplitudes) +
+                 (tr->n_traces > 0 ? ((tr->n_traces - 1) * tr->amp_row_stride + tr->n_samples) *
+                                         (int64_t)amp_elem_bytes(tr->amp_dtype) : 0);
     P.amp_stride = tr->amp_row_stride;
     P.n_traces = tr->n_traces;
     P.ns = tr->n_samples;
@@ -88,7 +91,7 @@ inline KParams make_params(const pstm_traces_desc *tr, const pstm_output_desc *o
     P.s_rej_lo = -g;
     P.s_rej_hi = smax + g;
     P.s_max_clamp = std::nextafter(smax, 0.0f);
-    P.s_magic = 2147483648.0 - P.tstart_s / P.dt_s;
+    P.s_magic = (kIndexMagic - P.tstart_s / P.dt_s) * kTimeScale;
     P.inv_dt_f = (float)(1.0 / P.dt_s);
 
     P.image = out->image;
@@ -111,7 +114,6 @@ inline KParams make_params(const pstm_traces_desc *tr, const pstm_output_desc *o
     P.tan_dip = std::tan(prm->max_dip_degrees * M_PI / 180.0);
     P.taper = prm->taper_fraction;
     P.fold_d2_max = sqrt_threshold(prm->max_aperture_m);
-    P.ap_max_f = (float)prm->max_aperture_m;
     P.taper_f = (float)prm->taper_fraction;
     P.spreading = prm->apply_spreading ? 1 : 0;
     P.obliquity = prm->apply_obliquity ? 1 : 0;
@@ -123,15 +125,14 @@ inline KParams make_params(const pstm_traces_desc *tr, const pstm_output_desc *o
     P.aa_fdom = prm->aa_dominant_freq;
     P.cr_v0 = prm->curved_v0;
     P.cr_k = prm->curved_k;
-    P.cr_v0f = (float)prm->curved_v0;
-    P.cr_kf = (float)prm->curved_k;
     P.cr_k_zero = std::fabs(prm->curved_k) < 1e-10 ? 1 : 0;
     P.cr_inv_k_ln2 = P.cr_k_zero ? 0.f : (float)(M_LN2 / prm->curved_k);
     // VTI returns 2 t0/2 = 0 at t0 = 0; the curved leg of depth 0 is log(1) = 0 for k != 0
     P.t0_zero_exact = (prm->traveltime == PSTM_TT_VTI ||
                        ((prm->traveltime == PSTM_TT_CURVED || prm->traveltime == PSTM_TT_CURVED_VTI) &&
                         !P.cr_k_zero)) ? 1 : 0;
-    P.compensated = prm->compensated ? 1 : 0;
+    P.exact_units = prm->precision == PSTM_PREC_EXACT ? 1 : 0;
+    P.curved_kind = (prm->traveltime == PSTM_TT_CURVED || prm->traveltime == PSTM_TT_CURVED_VTI) ? 1 : 0;
     P.cr_B0 = 1.0 / (prm->curved_v0 * prm->curved_v0 * P.dt_s * P.dt_s);
     P.cr_k2 = prm->curved_k * prm->curved_k;
     P.cr_inv_k_dt = P.cr_k_zero ? 0.0 : 1.0 / (prm->curved_k * P.dt_s);
@@ -147,56 +148,56 @@ inline KParams make_params(const pstm_traces_desc *tr, const pstm_output_desc *o
         }
     }
 
-    // pillar patch: PB pillars as px x py, favouring y (the fastest image axis)
-    int py = PB, px = 1;
-    while (py > 1 && py > out->ny) { py /= 2; px *= 2; }
-    if (py == PB && PB >= 4) { py = PB / 2; px = 2; }
-    P.px = px;
-    P.py = py;
-    P.n_pblk_y = (out->ny + py - 1) / py;
+    // Pillar patch: the px x py = kPillars rectangle that covers the tile with the
+    // fewest patches, 2 x 4 first (the closer its pillars, the shorter the sample
+    // ranges a CTA stages).
+    const int shapes[4][2] = {{2, 4}, {4, 2}, {1, 8}, {8, 1}};
+    int64_t best = -1;
+    for (const auto &sh : shapes) {
+        const int64_t nbx = (out->nx + sh[0] - 1) / sh[0], nby = (out->ny + sh[1] - 1) / sh[1];
+        if (best >= 0 && nbx * nby >= best) continue;
+        best = nbx * nby;
+        P.px = sh[0];
+        P.py = sh[1];
+        P.n_pblk_x = (int32_t)nbx;
+        P.n_pblk_y = (int32_t)nby;
+    }
+    P.n_tblk = (out->nt + kTimes - 1) / kTimes;
+    P.n_pblk_fold = (int32_t)(((int64_t)out->nx * out->ny + kFoldPillars - 1) / kFoldPillars);
+    P.max_chunk = kChunk;
+    // CTAs that share an item's traces: enough for two per SM four times over
+    // (148 SMs), by the tile's size alone, so that a bin and the same traces as
+    // a tile of their own are summed in the same order.
+    P.n_splits = 1;
+    while (P.n_splits < kMaxSplits && best * P.n_tblk * P.n_splits < 4 * 2 * 148) P.n_splits *= 2;
     return P;
 }
 
-
-// Output times per lane (R) and pillars per CTA (PB) for a tile; force_* > 0
-// override them (tuning).  amp_dtype: 16-bit rows stage twice the traces per
-// byte, and there 8 pillars per CTA amortise a chunk's staging, records and
-// barrier over twice the pairs (measured on the case-2 tile, 262,144 traces:
-// FP16 5 % faster with 8 than with 4 pillars, FP32 6 % slower).
-inline void choose_shape(int nt, int force_r, int force_pb, int &R, int &PB, int amp_dtype = PSTM_AMP_F32) {
-    R = (nt + kThreads - 1) / kThreads;   // the whole output trace in one CTA where it fits
+// The interface's limit on a trace row: two rows, the pillars' records and the
+// partial sums of up to 4096 output times in one SM's shared memory.
+inline bool row_fits(const pstm_traces_desc *tr, const pstm_params *prm, int nt, int smem_optin) {
+    int R = (nt + 511) / 512;
     if (R > 8) R = 8;
-    if (force_r >= 1 && force_r <= 8) R = force_r;
-    PB = (R <= 1 || amp_dtype != PSTM_AMP_F32) ? 8 : 4;
-    if (force_pb >= 1 && force_pb <= kMaxPB) PB = force_pb;
+    const int PB = (R <= 1 || tr->amp_dtype != PSTM_AMP_F32) ? 8 : 4;
+    const bool has_c = prm->traveltime == PSTM_TT_CURVED || prm->traveltime == PSTM_TT_CURVED_VTI;
+    const int64_t fixed = 4096 + (int64_t)PB * 1024 * (has_c ? 3 : 2) +
+                          (int64_t)PB * R * 512 * (prm->compensated ? 6 : 4) + 3072;
+    const int64_t eb = (int64_t)amp_elem_bytes(tr->amp_dtype), pitch = (tr->n_samples + 16 / eb - 1) / (16 / eb) * (16 / eb);
+    return smem_optin >= fixed + 2 * pitch * eb;
 }
 
-// Staging plan: row pitch, TMA eligibility, traces per chunk and the dynamic
-// shared memory of one CTA.  Returns false when a row does not fit.
-inline bool plan_staging(KParams &P, const pstm_traces_desc *tr, const pstm_params *prm, int PB, int R,
-                         int smem_optin, size_t &smem, int force_chunk = 0) {
-    const int eb = P.elem;
-    const int per16 = 16 / eb;
-    const int pitch = (tr->n_samples + per16 - 1) / per16 * per16;
-    const bool aligned = ((uintptr_t)tr->amplitudes % 16 == 0) && ((tr->amp_row_stride * eb) % 16 == 0);
-    P.pitch = pitch;
-    P.bulk = (aligned && tr->amp_row_stride >= pitch) ? 1 : 0;
-    const bool has_c = prm->traveltime == PSTM_TT_CURVED || prm->traveltime == PSTM_TT_CURVED_VTI;
-    const size_t fixed = 2 * (size_t)geo_buffer_bytes() + 2 * (size_t)record_buffer_bytes(PB, has_c) +
-                         (size_t)partial_bytes(PB, R, prm->compensated != 0);
-    const size_t static_bytes = 3072;   // s_ox/s_oy/s_pid/s_fold/s_rank/barriers, rounded up
-    const size_t budget = (size_t)smem_optin > fixed + static_bytes ? smem_optin - fixed - static_bytes : 0;
-    int chunk = (int)(budget / (2 * (size_t)pitch * eb));
-    if (chunk > kMaxChunk) chunk = kMaxChunk;
-    if (force_chunk >= 1 && force_chunk < chunk) chunk = force_chunk;   // tuning: a shallower panel
-    if (chunk < 1) return false;
-    P.chunk = chunk;
-    P.pb = PB;
-    P.r_per_lane = R;
-    P.flush_every = 16;
-    P.n_tblk = (P.nt + kThreads * R - 1) / (kThreads * R);
-    smem = 2 * (size_t)chunk * pitch * eb + fixed;
+// Grid of the gather kernel for `n_out` outputs of this tile: items x splits,
+// then the fold-counting CTAs, in whole clusters.  False: too many for one launch.
+inline bool plan_grid(const KParams &P, int64_t n_out, unsigned &grid) {
+    const int64_t items = (int64_t)P.n_pblk_x * P.n_pblk_y * P.n_tblk * n_out * P.n_splits;
+    const int64_t folds = ((int64_t)P.n_pblk_fold * n_out + P.n_splits - 1) / P.n_splits * P.n_splits;
+    if (items + folds > 0x7fffffff) return false;
+    grid = (unsigned)(items + folds);
     return true;
+}
+
+inline size_t gather_smem(int traveltime) {
+    return (size_t)dynamic_bytes(traveltime != PSTM_TT_STRAIGHT);
 }
 
 }  // namespace plan

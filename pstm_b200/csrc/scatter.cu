@@ -4,7 +4,7 @@
 // gives every trace one thread that walks the output points inside its
 // maximum aperture and adds one atomic per (point, sample); each trace is then
 // read once for the whole grid instead of once per tile whose selection box it
-// falls in.  Here the same decomposition runs on the gather machinery:
+// falls in.  Here the same decomposition runs on the gather kernel:
 //
 //   * the panel (any order; midpoint order keeps the segments compact) is cut
 //     into segments of S traces;
@@ -12,13 +12,11 @@
 //     bounding box, grows it by the maximum aperture and finds the pillar
 //     index ranges it covers by binary search in the grid axes, then the
 //     pillar blocks and the number of (pillar block, time block) items;
-//   * scan_counts turns the counts into inclusive prefix sums, on the device,
-//     so nothing is read back before the launch;
-//   * one persistent launch takes items from a work counter; an item finds its
-//     segment by binary search in the prefix sums and migrates the segment's
-//     traces against one pillar block and one time block, with the partial
-//     sums of the gather kernel (FP32 per chunk in shared memory) and one
-//     atomic add per output sample per item -- not one per pair.
+//   * one launch over the whole grid: a CTA (pillar block, time block) walks
+//     the segments whose boxes hold its block, 32 boxes at a time, and sums
+//     their traces in registers -- no atomics on the image;
+//   * scan_counts turns the counts into inclusive prefix sums when the caller
+//     asks for the number of items.
 //
 // Pillars outside a segment's box are farther than the maximum aperture from
 // every midpoint of the segment, so they receive nothing from it: image and
@@ -152,16 +150,15 @@ extern "C" int32_t pstm_cuda_migrate_scatter_dev(void *ctx, const pstm_traces_de
     int32_t rc = prepare_tile(c, traces, output, velocity, params, st, tp);
     if (rc || tp.empty) return rc;
     const KParams &P = tp.P;
-    // segments: a multiple of the staged chunk depth; default 64 chunks
-    int64_t S = segment_traces > 0 ? segment_traces : 64 * (int64_t)P.chunk;
-    S = (S + P.chunk - 1) / P.chunk * P.chunk;
+    // segments: whole chunks; default 64 chunks
+    int64_t S = segment_traces > 0 ? segment_traces : 64 * (int64_t)kChunk;
+    S = (S + kChunk - 1) / kChunk * kChunk;
     const int64_t n_seg = (P.n_traces + S - 1) / S;
     cudaError_t e;
-    if ((e = ensure(c->seg_bins, (size_t)n_seg * sizeof(SegmentBox))) != cudaSuccess ||
-        (e = ensure(c->scatter_ends, (size_t)n_seg * sizeof(long long))) != cudaSuccess ||
-        (e = ensure(c->seg_counter, sizeof(unsigned long long))) != cudaSuccess)
+    if ((e = ensure(c->seg_boxes, (size_t)n_seg * sizeof(SegmentBox))) != cudaSuccess ||
+        (e = ensure(c->scatter_ends, (size_t)n_seg * sizeof(long long))) != cudaSuccess)
         return cuda_fail(c, e, "allocating the scatter schedule");
-    SegmentBox *boxes = reinterpret_cast<SegmentBox *>(c->seg_bins.ptr);
+    SegmentBox *boxes = reinterpret_cast<SegmentBox *>(c->seg_boxes.ptr);
     long long *ends = reinterpret_cast<long long *>(c->scatter_ends.ptr);
     // a pillar farther than max_aperture (1 + 1e-9) + 1 um from every midpoint
     // of the segment is beyond the FP64 fold and aperture tests of them all
@@ -174,20 +171,14 @@ extern "C" int32_t pstm_cuda_migrate_scatter_dev(void *ctx, const pstm_traces_de
                                                         n_seg, output->x_axis, output->nx, output->y_axis,
                                                         output->ny, reach, P.px, P.py, P.n_tblk, boxes, ends, P.err);
         if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "segment_boxes launch");
-        scan_counts<<<1, kScanThreads, 0, st>>>(ends, n_seg);
-        if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "scan_counts launch");
+        if (n_items_out) {
+            scan_counts<<<1, kScanThreads, 0, st>>>(ends, n_seg);
+            if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "scan_counts launch");
+        }
     }
-    if ((e = cudaMemsetAsync(c->seg_counter.ptr, 0, sizeof(unsigned long long), st)) != cudaSuccess)
-        return cuda_fail(c, e, "clearing the work counter");
-    KParams Pa = P;
-    Pa.atomic_flush = 1;
-    Launch L;
-    L.smem = tp.L.smem;
-    L.stream = st;
-    L.counter = reinterpret_cast<unsigned long long *>(c->seg_counter.ptr);
-    L.scatter = ScatterWork{boxes, ends, n_seg, S};
-    e = launch_kind(tp.tt, Pa, tp.Pg, tp.amp, tp.per_pillar, tp.prec, L);
-    if (e != cudaSuccess) return cuda_fail(c, e, "scatter migrate launch");
+    tp.P.boxes = boxes;
+    tp.P.seg_traces = S;
+    if ((rc = launch_tile(c, tp)) != PSTM_OK) return rc;
     if (n_items_out) {   // diagnostics: the schedule's item count (synchronises the stream)
         long long total = 0;
         if ((e = cudaMemcpyAsync(&total, ends + (n_seg - 1), sizeof(total), cudaMemcpyDeviceToHost, st)) !=

@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(256) eval_kernel(const float *__restrict__ prm
 // Random in-aperture (pillar, trace, time) pairs of the tile: |T_surrogate -
 // T_exact| in ms, or -1 for a draw outside the pair's aperture.
 template <int TT>
-__global__ void __launch_bounds__(256) probe_kernel(const KParams P, const KParams *__restrict__ Pg,
+__global__ void __launch_bounds__(256) probe_kernel(const __grid_constant__ KParams P,
                                                     const float *__restrict__ prm, mlp::Norm nrm, uint64_t seed,
                                                     int n_probe, float *err_ms) {
     __shared__ mlp::Weights w;
@@ -363,19 +363,18 @@ __global__ void __launch_bounds__(256) probe_kernel(const KParams P, const KPara
         const double ox = P.xg ? P.xg[p] : P.xa[ix], oy = P.yg ? P.yg[p] : P.ya[iy];
         TimeState ts;
         PtState s;
-        load_states<TT_STRAIGHT, false>(P, p, t, ts, s);
+        point_state<TT_STRAIGHT>(P, p, t, UNIT_SECONDS, ts, s);
         const double dxm = ox - P.mx[tr], dym = oy - P.my[tr];
         const bool act = (float)sqrt(dxm * dxm + dym * dym) <= s.ap;
-        const float4 tab = P.ttab[(P.vel3d || P.eta3d) ? (int64_t)p * P.nt + t : t];
         const float dxs = (float)(ox - P.sx[tr]), dys = (float)(oy - P.sy[tr]);
         const float dxr = (float)(ox - P.rx[tr]), dyr = (float)(oy - P.ry[tr]);
-        const float r[7] = {(float)(P.ta[t] / 1000.0), dxs, dys, dxr, dyr, 1.f / tab.z, tab.w};
+        const float r[7] = {(float)(P.ta[t] / 1000.0), dxs, dys, dxr, dyr, 1.f / (float)(1.0 / s.v), (float)s.eta};
         float f[7];
         normalise(nrm, r, f);
         const float y = warp_mlp32(w, f);
         const float ds2 = fmaf(dxs, dxs, dys * dys), dr2 = fmaf(dxr, dxr, dyr * dyr);
         const float Td = sqrt_approx(fmaf(ds2, s.iv2, ts.t0h2)) + sqrt_approx(fmaf(dr2, s.iv2, ts.t0h2));
-        const double Te = exact_traveltime<TT>(Pg, tr, p, t, ox, oy);
+        const double Te = exact_traveltime<TT>(&P, tr, p, t, ox, oy);
         const float Ts = ts.tz ? 0.f : Td + y * nrm.out_scale;   // t0 = 0: T = 0 exactly, as the exact kernel
         if (i < n_probe) err_ms[i] = act ? (float)(fabs((double)Ts - Te) * 1000.0) : -1.f;
     }
@@ -400,28 +399,26 @@ __global__ void __launch_bounds__(128) migrate_learned_kernel(const KParams P, c
     const int tc = tv ? t : P.nt - 1;
     TimeState ts;
     PtState s;
-    // the weight tables are in samples when the tile was prepared for the FP64
+    // the weights are in samples when the tile was prepared for the FP64
     // sample-index kernel (its exact fallback), else in seconds; T is in seconds
     const bool samples = P.exact_units != 0;
-    if (samples) load_states<TT_STRAIGHT, true>(P, p, t, ts, s);   // s.ap < 0 past the tile end
-    else load_states<TT_STRAIGHT, false>(P, p, t, ts, s);
+    point_state<TT_STRAIGHT>(P, p, tc, samples ? UNIT_SAMPLES : UNIT_SECONDS, ts, s);
+    if (!tv) s.ap = -1.f;
     const float tw = samples ? P.inv_dt_f : 1.f;   // T in the weights' unit
-    const float4 tab = P.ttab[(P.vel3d || P.eta3d) ? (int64_t)p * P.nt + tc : tc];
-    const float t0 = (float)(P.ta[tc] / 1000.0), v = 1.f / tab.z, eta = tab.w;
+    const float t0 = (float)(P.ta[tc] / 1000.0), v = 1.f / (float)(1.0 / s.v), eta = (float)s.eta;
     const bool w_one = P.spreading + P.obliquity == 1, w_two = P.spreading + P.obliquity == 2;
     const float smax = (float)(P.ns - 1);
     float acc = 0.f;
     int cnt = 0;
     for (int64_t tr = 0; tr < P.n_traces; ++tr) {
-        const double *g = P.geo + tr * kGeoDoubles;
-        const double dxm = ox - g[4], dym = oy - g[5];
+        const double dxm = ox - P.mx[tr], dym = oy - P.my[tr];
         const double d2 = dxm * dxm + dym * dym;
         cnt += d2 <= P.fold_d2_max;
         const float d = (float)sqrt(d2);
         const bool act = tv && d <= s.ap;
         if (__any_sync(0xffffffffu, act)) {
-            const float dxs = (float)(ox - g[0]), dys = (float)(oy - g[1]);
-            const float dxr = (float)(ox - g[2]), dyr = (float)(oy - g[3]);
+            const float dxs = (float)(ox - P.sx[tr]), dys = (float)(oy - P.sy[tr]);
+            const float dxr = (float)(ox - P.rx[tr]), dyr = (float)(oy - P.ry[tr]);
             const float r[7] = {t0, dxs, dys, dxr, dyr, v, eta};
             float f[7];
             normalise(nrm, r, f);
@@ -439,7 +436,7 @@ __global__ void __launch_bounds__(128) migrate_learned_kernel(const KParams P, c
                 reinterpret_cast<const unsigned char *>(P.amps) + (tr * P.amp_stride) * (int64_t)P.elem;
             const float a0 = amp_at<AMP>(row, i0), a1 = amp_at<AMP>(row, ok ? i0 + 1 : 0);
             const float amp = fmaf(fr, a1 - a0, a0);
-            float wt = ok ? (float)g[6] : 0.f;
+            float wt = ok ? (P.w ? (float)P.w[tr] : 1.f) : 0.f;
             const float x = fmaf(d, s.itw, s.tsn);
             wt *= x > 0.f ? taper_weight(x) : 1.f;
             const float Tw = T * tw;
@@ -594,9 +591,9 @@ int32_t pstm_cuda_migrate_tile_learned_dev(void *ctx, const pstm_traces_desc *tr
     const mlp::Norm nrm = to_norm(net);
     const uint64_t seed = 0x5EED5EEDull ^ (uint64_t)tp.P.n_traces;
     if (tp.tt == PSTM_TT_VTI)
-        probe_kernel<TT_VTI><<<grid_for(n_probe, 256), 256, 0, st>>>(tp.P, tp.Pg, net->params, nrm, seed, n_probe, err);
+        probe_kernel<TT_VTI><<<grid_for(n_probe, 256), 256, 0, st>>>(tp.P, net->params, nrm, seed, n_probe, err);
     else
-        probe_kernel<TT_CURVED_VTI><<<grid_for(n_probe, 256), 256, 0, st>>>(tp.P, tp.Pg, net->params, nrm, seed,
+        probe_kernel<TT_CURVED_VTI><<<grid_for(n_probe, 256), 256, 0, st>>>(tp.P, net->params, nrm, seed,
                                                                             n_probe, err);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "probe launch");
     std::string host(n_probe * sizeof(float), '\0');

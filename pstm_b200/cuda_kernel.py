@@ -674,7 +674,7 @@ def _batch_descs(kernel: "CudaKernel", traces, bins, geometry, velocity, config,
 
 def migrate_bins(kernel: "CudaKernel", traces, bins, geometry, velocity, config=None,
                  kernel_type: str = "straight_ray") -> KernelMetrics:
-    """Migrate many bins sharing one tile geometry in ONE persistent launch
+    """Migrate many bins sharing one tile geometry in ONE launch
     (replayed from a CUDA graph while the arguments repeat).
 
     ``traces`` holds every bin's traces (CUDA tensors), ``bins`` is a list of
