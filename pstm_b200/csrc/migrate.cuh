@@ -315,7 +315,7 @@ __device__ __forceinline__ double record_square(double x) {
 // 3.4 issue cycles) and no velocity in the weights.
 // CLAMP: radicands that odd parameters (eta < -0.15) can push below zero are
 // kept above it.
-template <int TT, bool CLAMP>
+template <int TT, bool KZ, bool CLAMP>
 __device__ __forceinline__ double exact_time(const KParams &P, const XState &x, bool tz, bool tzero, const double2 &B,
                                              const double2 &C, double &v) {
     const double magic = P.s_magic;
@@ -340,7 +340,7 @@ __device__ __forceinline__ double exact_time(const KParams &P, const XState &x, 
         return T;
     } else if constexpr (TT == TT_CURVED) {   // |k| ~ 0: straight rays in v0 (curved_ray.py:35-38)
         double T;
-        if (P.cr_k_zero) {
+        if constexpr (KZ) {
             T = (sqrt_newton(fma(B.x, P.cr_B0, x.A)) + sqrt_newton(fma(B.y, P.cr_B0, x.A))) * kTimeScale;
         } else {
             const double as = x.vz + sqrt_newton(fma(P.cr_k2, B.x, x.vz2));
@@ -352,7 +352,7 @@ __device__ __forceinline__ double exact_time(const KParams &P, const XState &x, 
         return T;
     } else {
         double tcs, tcr;
-        if (P.cr_k_zero) {
+        if constexpr (KZ) {
             tcs = sqrt_newton(fma(B.x, P.cr_B0, x.A)) * kTimeScale;
             tcr = sqrt_newton(fma(B.y, P.cr_B0, x.A)) * kTimeScale;
         } else {
@@ -370,7 +370,8 @@ __device__ __forceinline__ double exact_time(const KParams &P, const XState &x, 
             ur = fmax(ur, 1e-40);
         }
         double T = fma(tcs, sqrt_newton(us), tcr * sqrt_newton(ur));
-        if (tzero) T = tz ? 0.0 : tcs + tcr;   // t0 = 0: nothing, or (|k| ~ 0) the curved legs alone
+        if constexpr (CLAMP || KZ)   // t0 = 0: nothing, or (|k| ~ 0, where no point is odd) the curved legs alone
+            T = tzero ? (tz ? 0.0 : tcs + tcr) : T;
         v = T + magic;
         return T;
     }
@@ -490,29 +491,28 @@ static __device__ __noinline__ bool exact_outside_aperture(const KParams *P, int
 // ---------------------------------------------------------------- traveltime (FP32)
 // B = {ds2, dr2, k^2 ds2 | ds2^2, k^2 dr2 | dr2^2}; C (curved kinds) =
 // {1/(bs br) | 1/bs, 1/br, ds2^2, dr2^2}.  Result in seconds.
-template <int TT>
+// KZ: |k| < 1e-10, straight rays in v0 for the curved leg.  TESTS: points at t0 = 0
+// are possible (the EDGE loop); without it no lane branches.
+template <int TT, bool KZ, bool TESTS>
 __device__ __forceinline__ float traveltime(const KParams &P, const TimeState &ts, const PtState &s,
                                             const float4 &B, const float4 &Cc) {
-    if constexpr (TT == TT_STRAIGHT) {
+    if constexpr (TT == TT_STRAIGHT || (TT == TT_CURVED && KZ)) {
         return sqrt_approx(fmaf(B.x, s.iv2, ts.t0h2)) + sqrt_approx(fmaf(B.y, s.iv2, ts.t0h2));
     } else if constexpr (TT == TT_CURVED) {
-        if (P.cr_k_zero) {
-            return sqrt_approx(fmaf(B.x, s.iv2, ts.t0h2)) + sqrt_approx(fmaf(B.y, s.iv2, ts.t0h2));
-        }
         const float a = ts.vz + sqrt_approx(ts.vz2 + B.z);
         const float b = ts.vz + sqrt_approx(ts.vz2 + B.w);
         return P.cr_inv_k_ln2 * lg2_approx(a * b * Cc.x);
     } else if constexpr (TT == TT_VTI) {
-        if (ts.tzero) return 0.f;
         const float Ds = fmaf(s.c1, B.x, s.t02v2);
         const float Dr = fmaf(s.c1, B.y, s.t02v2);
         const float rr = rcp_approx(Ds * Dr);
         const float qs = fmaf(-(s.e2 * B.z), Dr * rr, fmaf(B.x, s.iv2, ts.t0h2));
         const float qr = fmaf(-(s.e2 * B.w), Ds * rr, fmaf(B.y, s.iv2, ts.t0h2));
-        return sqrt_approx(fmaxf(qs, 0.f)) + sqrt_approx(fmaxf(qr, 0.f));
+        const float T = sqrt_approx(fmaxf(qs, 0.f)) + sqrt_approx(fmaxf(qr, 0.f));
+        return TESTS && ts.tzero ? 0.f : T;
     } else {
         float tcs, tcr;
-        if (P.cr_k_zero) {
+        if constexpr (KZ) {
             tcs = sqrt_approx(fmaf(B.x, s.iv2, ts.t0h2));
             tcr = sqrt_approx(fmaf(B.y, s.iv2, ts.t0h2));
         } else {
@@ -521,14 +521,14 @@ __device__ __forceinline__ float traveltime(const KParams &P, const TimeState &t
             tcs = P.cr_inv_k_ln2 * lg2_approx(a * Cc.x);
             tcr = P.cr_inv_k_ln2 * lg2_approx(b * Cc.y);
         }
-        if (ts.tzero) return tcs + tcr;
         // leg = t_curved * sqrt(1 - corr / (t0h^2 + h^2/v^2)), corr = e2 h^4 / D, v = v_rms
         const float Hs = fmaf(B.x, s.iv2r, ts.t0h2), Hr = fmaf(B.y, s.iv2r, ts.t0h2);
         const float Ds = fmaf(s.c1, B.x, s.t02v2), Dr = fmaf(s.c1, B.y, s.t02v2);
         const float ps_ = Ds * Hs, pr_ = Dr * Hr;
         const float rr = rcp_approx(ps_ * pr_);
         const float xs = s.e2 * Cc.z * (pr_ * rr), xr = s.e2 * Cc.w * (ps_ * rr);
-        return tcs * sqrt_approx(fmaxf(1.f - xs, 0.f)) + tcr * sqrt_approx(fmaxf(1.f - xr, 0.f));
+        const float T = tcs * sqrt_approx(fmaxf(1.f - xs, 0.f)) + tcr * sqrt_approx(fmaxf(1.f - xr, 0.f));
+        return TESTS && ts.tzero ? tcs + tcr : T;
     }
 }
 
@@ -703,7 +703,8 @@ __device__ __forceinline__ float amp_global(const KParams &P, long long id, int 
 // ---------------------------------------------------------------- the kernel
 // W2: spreading and obliquity both on (the common case), else the weight
 // exponent is chosen at run time.  AA: the triangle antialiasing weight.
-template <int TT, int PREC, bool W2, bool AA>
+// KZ: curved kinds with |k| < 1e-10 (straight rays in v0).
+template <int TT, int PREC, bool W2, bool AA, bool KZ>
 __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_constant__ KParams P) {
     namespace cg = cooperative_groups;
     constexpr bool EXACT = PREC == PSTM_PREC_EXACT;
@@ -1112,7 +1113,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                 double2 Cd = make_double2(0.0, 0.0);
                 if constexpr (HAS_C) Cd = *reinterpret_cast<const double2 *>(r + RC);
                 double v;
-                const double T2 = exact_time<TT, decltype(clamp_c)::value>(P, xs[g], ts[g].tz, ts[g].tzero, B, Cd, v);
+                const double T2 = exact_time<TT, KZ, decltype(clamp_c)::value>(P, xs[g], ts[g].tz, ts[g].tzero, B, Cd, v);
                 word = (unsigned)__double2hiint(v);
                 f = __uint_as_float(__funnelshift_r((unsigned)__double2loint(v), 0x7Fu, 9));
                 T = scaled_double_to_float(T2);
@@ -1121,7 +1122,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                 const float4 B = *reinterpret_cast<const float4 *>(r);
                 float4 Cf = make_float4(0.f, 0.f, 0.f, 0.f);
                 if constexpr (CURVED) Cf = *reinterpret_cast<const float4 *>(r + RC);
-                T = traveltime<TT>(P, ts[g], st[g], B, Cf);
+                T = traveltime<TT, KZ, (decltype(clamp_c)::value || KZ)>(P, ts[g], st[g], B, Cf);
                 const float s = fmaf(T, s_scale, s_offset);
                 const float fl = __fadd_rd(s, 8388608.f);
                 word = (unsigned)__float_as_int(fl);

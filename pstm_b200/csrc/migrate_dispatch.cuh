@@ -33,9 +33,9 @@ static cudaError_t opt_in_smem(SmemOptIn &state, Kernel kern, size_t smem) {
     return e;
 }
 
-template <int TT, int PREC, bool W2, bool AA>
+template <int TT, int PREC, bool W2, bool AA, bool KZ>
 static cudaError_t launch_one(const KParams &P, const Launch &L) {
-    auto kern = gather_kernel<TT, PREC, W2, AA>;
+    auto kern = gather_kernel<TT, PREC, W2, AA, KZ>;
     static SmemOptIn opt_in;   // per instantiation
     cudaError_t e = opt_in_smem(opt_in, kern, L.smem);
     if (e != cudaSuccess || L.configure_only) return e;
@@ -55,11 +55,18 @@ static cudaError_t launch_one(const KParams &P, const Launch &L) {
     return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
+template <int TT, int PREC, bool KZ>
+static cudaError_t launch_weights(const KParams &P, const Launch &L) {
+    const bool w2 = P.spreading && P.obliquity;
+    if (P.aa) return w2 ? launch_one<TT, PREC, true, true, KZ>(P, L) : launch_one<TT, PREC, false, true, KZ>(P, L);
+    return w2 ? launch_one<TT, PREC, true, false, KZ>(P, L) : launch_one<TT, PREC, false, false, KZ>(P, L);
+}
+
 template <int TT, int PREC>
 static cudaError_t launch_prec(const KParams &P, const Launch &L) {
-    const bool w2 = P.spreading && P.obliquity;
-    if (P.aa) return w2 ? launch_one<TT, PREC, true, true>(P, L) : launch_one<TT, PREC, false, true>(P, L);
-    return w2 ? launch_one<TT, PREC, true, false>(P, L) : launch_one<TT, PREC, false, false>(P, L);
+    if constexpr (TT == TT_CURVED || TT == TT_CURVED_VTI)
+        if (P.cr_k_zero) return launch_weights<TT, PREC, true>(P, L);
+    return launch_weights<TT, PREC, false>(P, L);
 }
 
 template <int TT>
