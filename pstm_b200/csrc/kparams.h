@@ -95,7 +95,7 @@ struct KParams {
     int32_t *err;                // device error word (KernelError bits)
     double cr_B0;                // 1 / (v0 dt)^2: |k| ~ 0 straight rays in v0
     double cr_k2;                // k^2
-    double cr_inv_k_dt;          // 1 / (k dt)
+    double cr_inv_k_dt;          // kTimeScale / (k dt)
     int32_t wait_iters;          // polls of one bounded mbarrier wait before it gives up
     int32_t inject_stall;        // fault injection: the first chunks' copies are never issued, so the
                                  // bounded waits for them run out (host-selected, tests only)

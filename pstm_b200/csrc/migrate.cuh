@@ -50,6 +50,7 @@
 #include <type_traits>
 
 #include "kparams.h"
+#include "logtab.cuh"
 #include "pstm_cuda.h"
 
 namespace pstm {
@@ -279,34 +280,44 @@ __device__ __forceinline__ void point_state(const KParams &P, int p, int t, int 
 }
 
 // The FP64 numbers of one point that the EXACT pair loop keeps: C = (t0 v / 2)^2
-// (times kQScale but for curved+VTI's ratio), iv = 1 / (v dt), c1 = 1 + 2 eta,
-// e2 = 2 eta, v(z) and its square.
+// (times kQScale, or k^2 for curved+VTI), iv = 1 / (v dt), c1 = 1 + 2 eta, e2 = 2 eta,
+// 2 v(z) and v(z)^2.
 struct XState {
     double A, C, iv, c1, e2, vz, vz2;
 };
-template <int TT>
+template <int TT, bool KZ>
 __device__ __forceinline__ XState exact_state(const KParams &P, const TimeState &ts, const PtState &s) {
+    constexpr bool CURVED = TT == TT_CURVED || TT == TT_CURVED_VTI;
     XState x;
     x.A = ts.A;
-    x.C = ts.A / s.B * ((TT == TT_STRAIGHT || TT == TT_VTI) ? kQScale : 1.0);
+    x.C = ts.A / s.B * (CURVED ? (KZ ? 1.0 : P.cr_k2) : kQScale);
     x.iv = 1.0 / (s.v * P.dt_s);
     x.c1 = 1.0 + 2.0 * s.eta;
     x.e2 = 2.0 * s.eta;
-    x.vz = ts.vz64;
+    x.vz = 2.0 * ts.vz64;
     x.vz2 = ts.vz64 * ts.vz64;
     return x;
 }
-// The squared distances of an EXACT record: straight and VTI carry them times kQScale.
-template <int TT>
-__device__ __forceinline__ double record_square(double x) {
-    if constexpr (TT != TT_STRAIGHT && TT != TT_VTI) return x;
+// The squared distances h^2 of an EXACT record: straight and VTI carry them times
+// kQScale, the curved kinds times k^2.
+template <int TT, bool KZ>
+__device__ __forceinline__ double record_square(const KParams &P, double x) {
+    if constexpr (TT == TT_CURVED || TT == TT_CURVED_VTI) return KZ ? x : P.cr_k2 * x;
     // x 2^254 by the exponent (x = 0 becomes 2^-769: as good as 0 beside C)
     return __hiloint2double(__double2hiint(x) + (254 << 20), __double2loint(x));
 }
+// Twice v + sqrt(v^2 + k^2 h^2), the numerator of a curved leg's logarithm.
+__device__ __forceinline__ double curved_numerator(const XState &x, double kx) {
+    const double q = kx + x.vz2;
+    double h;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(h) : "d"(q));
+    const double w = q * h;
+    return fma(w, fma(-w, h, 3.0), x.vz);
+}
 
 // FP64 traveltime (the EXACT path) of one pair from its record: B = {ds2, dr2},
-// C = VTI {ds2^2, dr2^2}, curved {1/(bs br), 0} or curved+VTI {1/bs, 1/br}, bs =
-// v0 + sqrt(v0^2 + k^2 ds2).  Returns T times 2^128 in the weights' unit and puts
+// C = VTI {ds2^2, dr2^2}, curved {1/(4 bs br), 0} or curved+VTI {1/(2 bs), 1/(2 br)},
+// bs = v0 + sqrt(v0^2 + k^2 ds2).  Returns T times 2^128 in the weights' unit and puts
 // the sample index word into `v`: the sum of 2^20 + index, times 2^128.
 // Straight and VTI work in metres: a leg's effective length is sqrt(C + x) with
 // x = h^2, and with the VTI correction sqrt(C + x - 2 eta x^2 / (C + (1+2eta) x)); the
@@ -316,8 +327,8 @@ __device__ __forceinline__ double record_square(double x) {
 // CLAMP: radicands that odd parameters (eta < -0.15) can push below zero are
 // kept above it.
 template <int TT, bool KZ, bool CLAMP>
-__device__ __forceinline__ double exact_time(const KParams &P, const XState &x, bool tz, bool tzero, const double2 &B,
-                                             const double2 &C, double &v) {
+__device__ __forceinline__ double exact_time(const KParams &P, const LogEntry *log_tab, const XState &x, bool tz,
+                                             bool tzero, const double2 &B, const double2 &C, double &v) {
     const double magic = P.s_magic;
     if constexpr (TT == TT_STRAIGHT || TT == TT_VTI) {
         double qs = B.x + x.C, qr = B.y + x.C, hs, hr;
@@ -339,27 +350,26 @@ __device__ __forceinline__ double exact_time(const KParams &P, const XState &x, 
         v = fma(T, x.iv, magic);
         return T;
     } else if constexpr (TT == TT_CURVED) {   // |k| ~ 0: straight rays in v0 (curved_ray.py:35-38)
-        double T;
         if constexpr (KZ) {
-            T = (sqrt_newton(fma(B.x, P.cr_B0, x.A)) + sqrt_newton(fma(B.y, P.cr_B0, x.A))) * kTimeScale;
+            const double T = (sqrt_newton(fma(B.x, P.cr_B0, x.A)) + sqrt_newton(fma(B.y, P.cr_B0, x.A))) * kTimeScale;
+            v = T + magic;
+            return T;
         } else {
-            const double as = x.vz + sqrt_newton(fma(P.cr_k2, B.x, x.vz2));
-            const double ar = x.vz + sqrt_newton(fma(P.cr_k2, B.y, x.vz2));
-            T = log(as * ar * C.x) * (P.cr_inv_k_dt * kTimeScale);
-            if constexpr (CLAMP) T = tz ? 0.0 : T;   // depth 0: both legs are log(1) = 0
+            double L = log_by_table(log_tab, curved_numerator(x, B.x) * curved_numerator(x, B.y) * C.x);
+            if constexpr (CLAMP) L = tz ? 0.0 : L;   // depth 0: both legs are log(1) = 0
+            v = fma(L, P.cr_inv_k_dt, magic);
+            return L * P.cr_inv_k_dt;
         }
-        v = T + magic;
-        return T;
     } else {
         double tcs, tcr;
         if constexpr (KZ) {
-            tcs = sqrt_newton(fma(B.x, P.cr_B0, x.A)) * kTimeScale;
-            tcr = sqrt_newton(fma(B.y, P.cr_B0, x.A)) * kTimeScale;
+            tcs = sqrt_newton(fma(B.x, P.cr_B0, x.A));
+            tcr = sqrt_newton(fma(B.y, P.cr_B0, x.A));
         } else {
-            tcs = log((x.vz + sqrt_newton(fma(P.cr_k2, B.x, x.vz2))) * C.x) * (P.cr_inv_k_dt * kTimeScale);
-            tcr = log((x.vz + sqrt_newton(fma(P.cr_k2, B.y, x.vz2))) * C.y) * (P.cr_inv_k_dt * kTimeScale);
+            tcs = log_by_table(log_tab, curved_numerator(x, B.x) * C.x);
+            tcr = log_by_table(log_tab, curved_numerator(x, B.y) * C.y);
         }
-        // leg = t_curved sqrt(1 - f), f = 2 eta x^2 / ((C + (1+2eta) x)(C + x))
+        // leg = t_curved sqrt(1 - f), f = 2 eta x^2 / ((C + (1+2eta) x)(C + x)), x and C times k^2
         const double Hs = B.x + x.C, Hr = B.y + x.C;
         const double Ds = fma(B.x, x.c1, x.C), Dr = fma(B.y, x.c1, x.C);
         const double ps = Ds * Hs, pr = Dr * Hr;
@@ -369,11 +379,12 @@ __device__ __forceinline__ double exact_time(const KParams &P, const XState &x, 
             us = fmax(us, 1e-40);
             ur = fmax(ur, 1e-40);
         }
-        double T = fma(tcs, sqrt_newton(us), tcr * sqrt_newton(ur));
+        double L = fma(tcs, sqrt_newton(us), tcr * sqrt_newton(ur));
         if constexpr (CLAMP || KZ)   // t0 = 0: nothing, or (|k| ~ 0, where no point is odd) the curved legs alone
-            T = tzero ? (tz ? 0.0 : tcs + tcr) : T;
-        v = T + magic;
-        return T;
+            L = tzero ? (tz ? 0.0 : tcs + tcr) : L;
+        const double unit = KZ ? kTimeScale : P.cr_inv_k_dt;
+        v = fma(L, unit, magic);
+        return L * unit;
     }
 }
 
@@ -713,8 +724,10 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
     constexpr bool HAS_C = TT != TT_STRAIGHT;
     constexpr int UNIT = !EXACT ? UNIT_SECONDS : (CURVED ? UNIT_SAMPLES : UNIT_METRES);
     constexpr unsigned INDEX_BASE = EXACT ? kHiBase : kFloatBase;
+    constexpr bool LOG = CURVED && EXACT && !KZ;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ CtaShared sh;
+    __shared__ LogEntry log_tab[LOG ? kLogEntries : 1];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool producer = warp == kPillars;
@@ -764,6 +777,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
     double *const sums = reinterpret_cast<double *>(edge_k + 2 * kConsumers);     // all [2][kConsumers]
     const uint32_t full0 = smem_u32(&sh.full[0]), full1 = smem_u32(&sh.full[1]);
     const uint32_t empty0 = smem_u32(&sh.empty[0]), empty1 = smem_u32(&sh.empty[1]);
+    if (LOG && tid < kLogEntries) log_tab[tid] = log_entry(tid);
     if (tid == kConsumers) {
         mbar_init(full0, 1);
         mbar_init(full1, 1);
@@ -798,7 +812,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
             const int t = tblk * kTimes + 32 * g + lane;
             const bool valid = t < P.nt;
             point_state<TT>(P, p, valid ? t : P.nt - 1, UNIT, ts[g], st[g]);
-            if (EXACT) xs[g] = exact_state<TT>(P, ts[g], st[g]);
+            if (EXACT) xs[g] = exact_state<TT, KZ>(P, ts[g], st[g]);
             const float A = (float)ts[g].A, B = (float)st[g].B, e = (float)st[g].eta, vz = ts[g].vz;
             bool fine = A < 1e30f && B > 0.f && B < 1e30f;
             if (TT == TT_VTI || TT == TT_CURVED_VTI) fine = fine && e >= -0.15f && e < 1e3f;
@@ -1113,7 +1127,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                 double2 Cd = make_double2(0.0, 0.0);
                 if constexpr (HAS_C) Cd = *reinterpret_cast<const double2 *>(r + RC);
                 double v;
-                const double T2 = exact_time<TT, KZ, decltype(clamp_c)::value>(P, xs[g], ts[g].tz, ts[g].tzero, B, Cd, v);
+                const double T2 = exact_time<TT, KZ, decltype(clamp_c)::value>(P, log_tab, xs[g], ts[g].tz, ts[g].tzero, B, Cd, v);
                 word = (unsigned)__double2hiint(v);
                 f = __uint_as_float(__funnelshift_r((unsigned)__double2loint(v), 0x7Fu, 9));
                 T = scaled_double_to_float(T2);
@@ -1368,7 +1382,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                 *reinterpret_cast<float4 *>(r + R1) = make_float4(mz, wt, __int_as_float(row.x), d);
                 *reinterpret_cast<int2 *>(rec + R2 + slot * 8) = make_int2(row.y, row.z);
                 if constexpr (EXACT) {
-                    const double xs2 = record_square<TT>(ds2), xr2 = record_square<TT>(dr2);
+                    const double xs2 = record_square<TT, KZ>(P, ds2), xr2 = record_square<TT, KZ>(P, dr2);
                     *reinterpret_cast<double2 *>(r) = make_double2(xs2, xr2);
                     if constexpr (TT == TT_VTI)
                         *reinterpret_cast<double2 *>(r + RC) = make_double2(xs2 * xs2, xr2 * xr2);
@@ -1381,7 +1395,8 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                     const double2 Cd = TT == TT_CURVED ? make_double2(rcp_newton(bs * br), 0.0)
                                                        : make_double2(rcp_newton(bs), rcp_newton(br));
                     if constexpr (EXACT) {
-                        *reinterpret_cast<double2 *>(r + RC) = Cd;
+                        *reinterpret_cast<double2 *>(r + RC) =
+                            TT == TT_CURVED ? make_double2(0.25 * Cd.x, 0.0) : make_double2(0.5 * Cd.x, 0.5 * Cd.y);
                     } else {
                         Bf.z = (float)(k2 * ds2);
                         Bf.w = (float)(k2 * dr2);
