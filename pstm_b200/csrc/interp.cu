@@ -22,6 +22,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <utility>
 
 #include "pstm_cuda.h"
 #include "kparams.h"
@@ -47,119 +48,164 @@ __device__ inline R sample_at(const unsigned char *row, int64_t i) {
     return (R)amp_at<AMP>(row, (int)i);
 }
 
-// sincospi in the interpolation arithmetic: FP64, or FP32 on the fast path.
-__device__ inline void sincospi_r(double x, double *s, double *c) { sincospi(x, s, c); }
-__device__ inline void sincospi_r(float x, float *s, float *c) { sincospif(x, s, c); }
 // 1/x in the interpolation arithmetic: the hardware approximation refined by
 // one Newton step in FP64 (~1 ulp), the approximation itself in FP32.
 __device__ inline double rcp_r(double x) { return rcp_newton(x); }
 __device__ inline float rcp_r(float x) { return rcp_approx(x); }
 
-// Nearest, Catmull-Rom cubic and linear interpolation at fractional index t
-// (0 <= t < ns - 1 is checked by the caller); linear also serves the wide
-// methods within their half-width of a trace end.
+// Nearest, Catmull-Rom cubic and linear interpolation at the fractional index i +
+// f, 0 <= f < 1 (0 <= i + f < ns - 1 is checked by the caller); linear also serves
+// the wide methods within their half-width of a trace end.
 // R is the arithmetic of the weights and taps: double (exact path) or float
-// (fast path); the sample index t is FP64 in both.
+// (fast path); the sample index is FP64 in both.
 template <int AMP, typename R>
-__device__ R interpolate_narrow(const unsigned char *row, int ns, double t, int method) {
-    if (method == PSTM_INTERP_NEAREST) {
-        const int64_t i = (int64_t)(t + 0.5);
-        return (i < 0 || i >= ns) ? R(0) : sample_at<AMP, R>(row, i);
-    }
-    if (method == PSTM_INTERP_CUBIC && t >= 1.0 && t < (double)(ns - 2)) {   // Catmull-Rom
-        const int64_t i = (int64_t)t;
-        const R u = (R)(t - (double)i);
+__device__ R interpolate_narrow(const unsigned char *row, int ns, int i, R f, int method) {
+    if (method == PSTM_INTERP_NEAREST) return sample_at<AMP, R>(row, f < R(0.5) ? i : i + 1);
+    if (method == PSTM_INTERP_CUBIC && i >= 1 && i < ns - 2) {   // Catmull-Rom
         const R p0 = sample_at<AMP, R>(row, i - 1), p1 = sample_at<AMP, R>(row, i);
         const R p2 = sample_at<AMP, R>(row, i + 1), p3 = sample_at<AMP, R>(row, i + 2);
         const R c3 = R(-0.5) * p0 + R(1.5) * p1 - R(1.5) * p2 + R(0.5) * p3;
         const R c2 = p0 - R(2.5) * p1 + R(2.0) * p2 - R(0.5) * p3;
         const R c1 = R(-0.5) * p0 + R(0.5) * p2;
-        return ((c3 * u + c2) * u + c1) * u + p1;
+        return ((c3 * f + c2) * f + c1) * f + p1;
     }
-    const int64_t i0 = (int64_t)t;
-    const R f = (R)(t - (double)i0);
-    return sample_at<AMP, R>(row, i0) * (R(1) - f) + sample_at<AMP, R>(row, i0 + 1) * f;
+    return sample_at<AMP, R>(row, i) * (R(1) - f) + sample_at<AMP, R>(row, i + 1) * f;
 }
 
-// Windowed sinc (LANCZOS false) or Lanczos (true) of half-width HW at
-// fractional index t, normalised by the sum of the weights; linear within HW
-// samples of a trace end.
-//
-// The taps need sin(pi x) and the sine or cosine of pi x / HW at x = frac - k,
-// k = -HW+1 .. HW.  Since sin(pi (frac - k)) = (-1)^k sin(pi frac) and the
-// window angle pi (frac - k) / HW moves by pi / HW from one tap to the next,
-// a chain of window angles carried by rotations through (cos_d, sin_d) =
-// (cos, sin)(pi / HW) gives every weight, and the factor sin(pi frac) common
-// to all taps cancels in the normalisation.  A rotation
-// adds about one rounding of a unit-sized value per tap (absolute 1e-15 after
-// 16 taps), harmless where the window enters as 0.5 (1 + cos).  Lanczos
-// divides sin(pi x / HW) by x, so it needs that sine accurate relative to its
-// size near x = 0: it runs two chains, each started by its own sincospi at a
-// tap beside x = 0 (k = 0 and k = 1) and carried outward.  The weights are
-// otherwise those of the direct formulas: sinc(x) = sin(pi x) / (pi x) with 1
-// for |x| < 1e-10, a Hann window 0.5 (1 + cos(pi x / HW)) that is 0 for
-// |x| >= HW, Lanczos sinc(x) sinc(x / HW).
-template <int AMP, int HW, bool LANCZOS, typename R>
-__device__ R interpolate_wide(const unsigned char *row, int ns, double t, R cos_d, R sin_d) {
-    if (t < (double)HW || t >= (double)(ns - HW)) {
-        const int64_t i0 = (int64_t)t;
-        const R f = (R)(t - (double)i0);
-        return sample_at<AMP, R>(row, i0) * (R(1) - f) + sample_at<AMP, R>(row, i0 + 1) * f;
+// cos(pi K / HW) and sin(pi K / HW) at compile time: the angle folded into
+// [0, pi / 2], then the Taylor series.
+constexpr double kPi = 3.14159265358979323846;
+constexpr double cx_cos(double x) {
+    double t = 1.0, s = 1.0;
+    for (int n = 1; n < 16; ++n) {
+        t *= -x * x / ((2.0 * n - 1.0) * (2.0 * n));
+        s += t;
     }
-    const int64_t ic = LANCZOS ? (int64_t)t : (int64_t)(t + 0.5);
-    const R frac = (R)(t - (double)ic);
-    // On a sample (|x| < 1e-10 at a tap: the tap's weight is 1 and the others'
-    // sin(pi x) factors vanish) the interpolant is that sample.
-    if (fabs(frac) < R(1e-10)) return sample_at<AMP, R>(row, ic);
-    if (LANCZOS && fabs(frac - R(1)) < R(1e-10)) return sample_at<AMP, R>(row, ic + 1);
-    // The factors common to every tap cancel in the normalisation, so they are
-    // left out: sinc weights sin(pi x_k) / (pi x_k) * 0.5 (1 + cos w_k) with
-    // sin(pi x_k) = (-1)^k sin(pi frac) become (-1)^k (1 + cos w_k) / x_k, and
-    // Lanczos weights sin(pi x_k) sin(pi x_k / HW) HW / (pi^2 x_k^2) become
-    // (-1)^k sin(pi x_k / HW) / x_k^2; one reciprocal per tap, no division.
-    R acc = R(0), norm = R(0);
-    auto tap = [&](int k, R sg, R s_w, R c_w) {
-        const int64_t i = ic + k;
-        if (i < 0 || i >= ns) return;   // (sinc rounds to the nearest sample: ic + HW can reach ns)
-        const R x = frac - (R)k;
-        const R rx = rcp_r(x);
-        R w;
-        if (LANCZOS) w = fabs(x) >= R(HW) ? R(0) : sg * s_w * rx * rx;
-        else w = fabs(x) >= R(HW) ? R(0) : sg * (R(1) + c_w) * rx;
-        acc += sample_at<AMP, R>(row, i) * w;
-        norm += w;
-    };
-    if (!LANCZOS) {   // one chain, k = -HW+1 .. HW, window angle dropping by pi / HW per tap
-        R s_w, c_w;
-        sincospi_r((frac + (R)(HW - 1)) * (R(1) / (R)HW), &s_w, &c_w);
-        R sg = ((HW - 1) & 1) ? R(-1) : R(1);
-#pragma unroll
-        for (int k = -HW + 1; k <= HW; ++k) {
-            tap(k, sg, s_w, c_w);
-            const R c_n = c_w * cos_d + s_w * sin_d;
-            s_w = s_w * cos_d - c_w * sin_d;
-            c_w = c_n;
-            sg = -sg;
-        }
-    } else {          // k = 0, -1, .., -HW+1 (angle growing), then k = 1, .., HW (angle dropping)
-#pragma unroll
-        for (int side = 0; side < 2; ++side) {
-            const R sin_a = side ? -sin_d : sin_d;
-            R s_w, c_w;
-            sincospi_r((frac - (R)side) * (R(1) / (R)HW), &s_w, &c_w);
-            R sg = side ? R(-1) : R(1);
-#pragma unroll
-            for (int n = 0; n < HW; ++n) {
-                tap(side ? 1 + n : -n, sg, s_w, c_w);
-                const R c_n = c_w * cos_d - s_w * sin_a;
-                s_w = s_w * cos_d + c_w * sin_a;
-                c_w = c_n;
-                sg = -sg;
-            }
-        }
-    }
-    return norm != R(0) ? acc * rcp_r(norm) : R(0);
+    return s;
 }
+constexpr double cx_fold(int k, int hw) {   // cos(pi k / hw), |k| <= 2 hw
+    if (k < 0) k = -k;
+    if (k > hw) k = 2 * hw - k;
+    if (2 * k == hw) return 0.0;
+    return 2 * k > hw ? -cx_cos(kPi * (hw - k) / hw) : cx_cos(kPi * k / hw);
+}
+template <int HW, int K>
+constexpr double win_cos = cx_fold(K, HW);
+template <int HW, int K>
+constexpr double win_sin = cx_fold(2 * K - HW, 2 * HW);   // cos of the angle less pi / 2
+constexpr double cx_inv_factorial(int n) {
+    double f = 1.0;
+    for (int i = 2; i <= n; ++i) f /= i;
+    return f;
+}
+template <int N>
+constexpr double taylor = (N / 2 % 2 ? -1.0 : 1.0) * cx_inv_factorial(N);   // of y^N in cos (even N) or sin
+// Taylor polynomial in u = y^2 from y^N on, up to the power LAST.
+template <int N, int LAST, typename R>
+__device__ __forceinline__ R taylor_from(R u) {
+    if constexpr (N + 2 > LAST) return (R)taylor<N>;
+    else return taylor_from<N + 2, LAST, R>(u) * u + (R)taylor<N>;
+}
+// Last power of y = pi f / HW that matters: the next one's term is below 2^-54.
+constexpr int taylor_last(double y) {
+    int n = 1;
+    double t = y;
+    while (t > 0x1p-54) t *= y / ++n;
+    return n;
+}
+
+// Windowed sinc (LANCZOS false) or Lanczos (true) of half-width HW at the
+// fractional index i + f (0 <= f < 1), normalised by the sum of the weights; linear
+// within HW samples of a trace end.
+//
+// The direct weights are, at the 2 HW taps x_k = f - k, k = -HW+1 .. HW, sinc(x) =
+// sin(pi x) / (pi x) times a Hann window 0.5 (1 + cos(pi x / HW)) that is 0 for |x| >=
+// HW, or (Lanczos) times sinc(x / HW).  sin(pi x_k) is (-1)^k sin(pi f), so every
+// factor common to the taps cancels in the normalisation and what is left is
+//   sinc     (-1)^k (1 + cos(pi x_k / HW)) / x_k
+//   Lanczos  (-1)^k sin(pi x_k / HW) / x_k^2.
+// cos and sin of pi (f - k) / HW are combinations of C, S = cos, sin(pi f / HW) with
+// compile-time factors: two Taylor polynomials serve all taps.  The divisions go
+// too: taps k and 1 - k are the roots of D_k = f^2 - f - k (k - 1), so 1 / x_k = x_{1-k} /
+// D_k, and multiplying all weights by the product of the D's (again common)
+// leaves x_{1-k} E_k, E_k the product of the other D's.  Nothing is divided but the
+// final sum; on a sample (f = 0) the sinc weights of the other taps are 0 by
+// themselves, the Lanczos weights all vanish and the sample is returned.
+//
+// The form before this one took a Newton-refined reciprocal, a rotation of the
+// window angle and a libm sincospi per sample: 1160 issue cycles a pair for sinc8
+// in FP64 (FP64 instructions take 2.1-3.4 cycles to issue).
+template <int AMP, int HW, bool LANCZOS, typename R>
+struct Wide {
+    static constexpr int kLast = taylor_last(kPi * (LANCZOS ? 1.0 : 0.5) / HW);
+
+    const unsigned char *row;
+    int i, i_max;
+    R f, C, S, acc, norm;
+    R E[HW];   // E[k - 1]: product of the D's but D_k
+
+    template <int K>
+    __device__ __forceinline__ void tap(bool live) {
+        const R sg = (K & 1) ? R(-1) : R(1);
+        const R e = E[K > 0 ? K - 1 : -K] * (f - (R)(1 - K));   // x_{1-K} E
+        R w;
+        if constexpr (LANCZOS) {
+            const R sn = S * (R)win_cos<HW, K> - C * (R)win_sin<HW, K>;
+            w = sg * sn * e * e;
+        } else {
+            const R cs = C * (R)win_cos<HW, K> + S * (R)win_sin<HW, K>;
+            w = (sg + sg * cs) * e;
+        }
+        int j = i + K;
+        if constexpr (K == HW && !LANCZOS) {   // beyond the window (and possibly the trace) for f < 0
+            w = live ? w : R(0);
+            j = min(j, i_max);
+        }
+        acc += sample_at<AMP, R>(row, j) * w;
+        norm += w;
+    }
+    template <int... K>
+    __device__ __forceinline__ void taps(std::integer_sequence<int, K...>, bool live) {
+        (tap<K - HW + 1>(live), ...);
+    }
+    __device__ __forceinline__ R run(const unsigned char *r, int ns, int i0, R f0) {
+        if (i0 < HW || i0 >= ns - HW) return sample_at<AMP, R>(r, i0) * (R(1) - f0) + sample_at<AMP, R>(r, i0 + 1) * f0;
+        row = r;
+        i_max = ns - 1;
+        i = i0;
+        f = f0;
+        if constexpr (LANCZOS) {
+            if (f < R(1e-10)) return sample_at<AMP, R>(row, i);
+            if (R(1) - f < R(1e-10)) return sample_at<AMP, R>(row, i + 1);
+        } else if (f >= R(0.5)) {   // sinc counts from the nearest sample: -0.5 <= f < 0.5
+            i += 1;
+            f -= R(1);
+        }
+        const R y = f * (R)(kPi / HW), u = y * y;
+        C = taylor_from<0, kLast, R>(u);
+        S = taylor_from<1, kLast, R>(u) * y;
+        const R g = f * f - f;
+        R D[HW];
+#pragma unroll
+        for (int k = 1; k <= HW; ++k) D[k - 1] = g - (R)(k * (k - 1));
+        // E by prefix and suffix products
+        R pre = R(1);
+#pragma unroll
+        for (int k = 0; k < HW; ++k) {
+            E[k] = pre;
+            pre *= D[k];
+        }
+        R suf = R(1);
+#pragma unroll
+        for (int k = HW - 1; k >= 0; --k) {
+            E[k] *= suf;
+            suf *= D[k];
+        }
+        acc = norm = R(0);
+        taps(std::make_integer_sequence<int, 2 * HW>{}, f >= R(0));
+        return norm != R(0) ? acc * rcp_r(norm) : R(0);
+    }
+};
 
 template <int TT>
 __device__ inline double tt_of(double t0, double ds2, double dr2, double v, double eta, double v0, double k) {
@@ -201,8 +247,6 @@ __global__ void __launch_bounds__(kInterpThreads, PSTM_INTERP_MIN_CTAS) migrate_
     const double taper_start = ap * (1.0 - P.taper);
     const double inv_taper_w = ap > taper_start ? 1.0 / (ap - taper_start) : 0.0;
     const double iv2 = 1.0 / (v * v), t0h2 = (t0 * 0.5) * (t0 * 0.5), inv_dt = 1.0 / P.dt_s;
-    R sin_d = R(0), cos_d = R(1);
-    if (HW > 0) sincospi_r(R(1) / (R)HW, &sin_d, &cos_d);
 
     Staged &S = S_all[warp];
     // Largest aperture over the warp's output times: a trace farther than it
@@ -256,9 +300,18 @@ __global__ void __launch_bounds__(kInterpThreads, PSTM_INTERP_MIN_CTAS) migrate_
             if (!(s >= 0.0 && s < (double)(P.ns - 1))) continue;
             const unsigned char *row =
                 reinterpret_cast<const unsigned char *>(P.amps) + ((int64_t)S.tr[j] * P.amp_stride) * (int64_t)P.elem;
+            // integer and fraction without conversions: s + 1.5 2^52 has the nearest
+            // integer in its low word
+            const double near = s + 6755399441055744.0;
+            int i0 = __double2loint(near);
+            double fr = s - (near - 6755399441055744.0);
+            if (fr < 0.0) {
+                i0 -= 1;
+                fr += 1.0;
+            }
             R amp;
-            if (HW > 0) amp = interpolate_wide<AMP, HW, LANCZOS, R>(row, P.ns, s, cos_d, sin_d);
-            else amp = interpolate_narrow<AMP, R>(row, P.ns, s, method);
+            if constexpr (HW > 0) amp = Wide<AMP, HW, LANCZOS, R>().run(row, P.ns, i0, (R)fr);
+            else amp = interpolate_narrow<AMP, R>(row, P.ns, i0, (R)fr, method);
             R w = (R)S.w[j];
             if (dj > taper_start) {
                 const R x = (R)((dj - taper_start) * inv_taper_w);
