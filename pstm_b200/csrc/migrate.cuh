@@ -15,8 +15,8 @@
 //             test of the pair loop is known to pass for every lane; MID, where
 //             only the aperture's taper and the trace ends are open; and EDGE,
 //             the rest.  Then they
-//             run the classes' pair loops and add the chunk's FP32 sums into
-//             FP64.  16-bit samples are first widened to FP32 in shared memory.
+//             run the classes' pair loops; every four chunks their FP32 sums
+//             go into FP64.  16-bit samples are first widened to FP32 in shared memory.
 // No warp waits for another consumer (except to widen), so uneven chunks and the
 // producer's memory latency are hidden; the first form, in which the eight warps
 // selected, staged and built in turn between CTA barriers, lost 12 % of its warp
@@ -63,6 +63,7 @@ constexpr int kChunk = 32;                  // traces per chunk, upper bound: on
 constexpr int kRowPitch = 256;              // staged samples per trace with 32 traces per chunk
 constexpr int kPool = kChunk * kRowPitch;   // staged samples of one buffer
 constexpr int kMaxSplits = 8;               // CTAs of a cluster that share an item's traces
+constexpr int kFlush = 4;                   // chunks whose FP32 sums are added into FP64 together
 constexpr int kFoldPillars = 8;             // pillars per fold-counting CTA
 constexpr int kWaitIters = 1 << 20;         // default bound of every mbarrier wait loop (KParams::wait_iters)
 
@@ -388,32 +389,30 @@ __device__ __forceinline__ double exact_time(const KParams &P, const LogEntry *l
     }
 }
 
-// 0.5 (1 + cos(pi x)) = cos^2(pi x / 2) for x in [0, 1]: Taylor series of cos
-// about 0 through y^12 (|error| < 7e-9 on y in [0, pi/2]), then squared.
+// 0.5 (1 + cos(pi x)) = cos^2(pi x / 2) for x in [0, 1]: cos as a polynomial in x^2
+// with value 1 at 0 and the least largest error on [0, 1] (2.4e-10, fitted by
+// reweighted least squares), then squared; 1.3e-7 in FP32, all of it rounding.
+// Taylor's series takes two more terms for 7e-9.
+constexpr float kTaper1 = -1.2337005390219158f, kTaper2 = 0.25366934998483653f, kTaper3 = -0.020862751638218144f,
+                kTaper4 = 9.17788771589905e-4f, kTaper5 = -2.3848339607722318e-5f;
 __device__ __forceinline__ float taper_weight(float x) {
-    const float y = 1.57079632679489662f * x;
-    const float u = y * y;
-    float c = 2.08767569878681e-9f;                 //  1/12!
-    c = fmaf(c, u, -2.75573192239859e-7f);          // -1/10!
-    c = fmaf(c, u, 2.48015873015873e-5f);           //  1/8!
-    c = fmaf(c, u, -1.38888888888889e-3f);          // -1/6!
-    c = fmaf(c, u, 4.16666666666667e-2f);           //  1/4!
-    c = fmaf(c, u, -0.5f);                          // -1/2!
+    const float u = x * x;
+    float c = kTaper5;
+    c = fmaf(c, u, kTaper4);
+    c = fmaf(c, u, kTaper3);
+    c = fmaf(c, u, kTaper2);
+    c = fmaf(c, u, kTaper1);
     c = fmaf(c, u, 1.0f);
     return c * c;
 }
-
 // The same for two x in [0, 1], in packed FP32 pairs.
 __device__ __forceinline__ float2 taper_weight2(float2 x) {
     auto two = [](float a) { return make_float2(a, a); };
-    const float2 y = __fmul2_rn(two(1.57079632679489662f), x);
-    const float2 u = __fmul2_rn(y, y);
-    float2 c = two(2.08767569878681e-9f);
-    c = __ffma2_rn(c, u, two(-2.75573192239859e-7f));
-    c = __ffma2_rn(c, u, two(2.48015873015873e-5f));
-    c = __ffma2_rn(c, u, two(-1.38888888888889e-3f));
-    c = __ffma2_rn(c, u, two(4.16666666666667e-2f));
-    c = __ffma2_rn(c, u, two(-0.5f));
+    const float2 u = __fmul2_rn(x, x);
+    float2 c = __ffma2_rn(two(kTaper5), u, two(kTaper4));
+    c = __ffma2_rn(c, u, two(kTaper3));
+    c = __ffma2_rn(c, u, two(kTaper2));
+    c = __ffma2_rn(c, u, two(kTaper1));
     c = __ffma2_rn(c, u, two(1.0f));
     return __fmul2_rn(c, c);
 }
@@ -635,6 +634,7 @@ struct CtaShared {
     } warp[kPillars];
     float apmax[kPillars], t_lo, t_hi;
     float zero[2];
+    long long selected[kChunk];   // the producer's own list
 };
 
 // ---------------------------------------------------------------- fold
@@ -978,8 +978,8 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
         for (;; ++j) {
             // ---- select: up to C traces near the patch, one per lane
             int cnt = 0;
-            long long id = 0;
             int batches = 1;   // 32 traces first: enough in a dense panel
+            __syncwarp();
             while (cnt < C) {
                 if (pos >= end) {
                     if (!next_range()) break;
@@ -1002,19 +1002,18 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                     // (fmax drops a NaN midpoint, so ask the midpoint itself)
                     const bool in = dx * dx + dy * dy <= reach2 && mx[u] == mx[u] && my[u] == my[u];
                     const unsigned b = __ballot_sync(full, in);
-                    const int room = C - cnt, n = min(__popc(b), room);
-                    // lane cnt + r takes the r-th set bit of b
-                    const int r = lane - cnt;
-                    const int bit = r >= 0 && r < n ? (int)__fns(b, 0, r + 1) : 0;
-                    if (r >= 0 && r < n) id = base + 32 * u + bit;
-                    cnt += n;
-                    if (__popc(b) > room) pos = base + 32 * u + (int)__fns(b, 0, room + 1);
-                    else pos = min(end, base + 32 * (u + 1));
+                    const int r = __popc(b & below), room = C - cnt;
+                    if (in && r < room) sh.selected[cnt + r] = base + 32 * u + lane;
+                    const unsigned over = __ballot_sync(full, in && r == room);   // the first one left for the next chunk
+                    pos = over ? base + 32 * u + __ffs(over) - 1 : min(end, base + 32 * (u + 1));
+                    cnt += min(__popc(b), room);
                 }
                 batches = 4;
             }
             // ---- geometry, window and copy of this lane's trace
             const bool have = lane < cnt;
+            __syncwarp();
+            const long long id = have ? sh.selected[lane] : 0;
             double sx = 0, sy = 0, rx = 0, ry = 0, mx = 0, my = 0, w = 1.0;
             if (have) {
                 sx = P.sx[id]; sy = P.sy[id];
@@ -1146,7 +1145,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
         };
         // A PLAIN or MID record at both of the lane's times: locate and read each,
         // then the interpolation and weights of both.  The point's factor K is
-        // left to the end of the chunk.  The AA weight max(0, 1 - max(min(u aa_k,
+        // left to the flush.  The AA weight max(0, 1 - max(min(u aa_k,
         // aaA), f_dom/500)) is clamp(1 - u aa_k, L, H) with L = max(0, 1 - aaA), H =
         // max(0, 1 - f_dom/500).  MID adds the taper and the test of the index;
         // what is outside reads two zeros.  WEIGHT: the traces have weights.
@@ -1271,6 +1270,12 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
         };
         using F = std::false_type;
         using Tr = std::true_type;
+        float2 acc = make_float2(0.f, 0.f), acc_e = acc;   // PLAIN and MID records' sums (without K), EDGE records'
+        auto flush = [&]() {
+            sums[tid] += (double)fmaf(acc.x, edge_k[tid].x, acc_e.x);
+            sums[kConsumers + tid] += (double)fmaf(acc.y, edge_k[kConsumers + tid].x, acc_e.y);
+            acc = acc_e = make_float2(0.f, 0.f);
+        };
         for (int k = 0;; ++k) {
             const int b = k & 1;
             timeout = __any_sync(full, !mbar_wait(b ? full1 : full0, (uint32_t)((k >> 1) & 1), P.wait_iters));
@@ -1328,7 +1333,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                     const double dxr = ox - tab.rx[lane], dyr = oy - tab.ry[lane];
                     ds2 = dxs * dxs + dys * dys;
                     dr2 = dxr * dxr + dyr * dyr;
-                    wt = (float)tab.w[lane];
+                    wt = P.w ? (float)tab.w[lane] : 1.f;
                     mz = (float)fmax(fabs(dxm), fabs(dym));
                     if (!(row.w & TRACE_DROP)) {
                         // T > 1 ms and sin(theta) >= 0.01 at every point of the warp
@@ -1413,22 +1418,26 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
             __syncwarp();
 
             // ---- pairs
-            float2 acc = make_float2(0.f, 0.f), acc_e = acc;
             const bool wide = tab.wide != 0;   // rare: a window of this chunk is too long to stage
             const bool weighted = P.w != nullptr;
             if (!wide) {
                 const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (weighted) {
-#pragma unroll 2
+#pragma unroll 4
                     for (int c = 0; c < np; ++c) fast_record(c, acc, none, none, F{}, Tr{});
                 } else {
-#pragma unroll 2
+#pragma unroll 4
                     for (int c = 0; c < np; ++c) fast_record(c, acc, none, none, F{}, F{});
                 }
                 if (np < nm) {
                     const float4 e0 = edge_a[tid], e1 = edge_a[kConsumers + tid];
+                    if (weighted) {
 #pragma unroll 2
-                    for (int c = np; c < nm; ++c) fast_record(c, acc, e0, e1, Tr{}, Tr{});
+                        for (int c = np; c < nm; ++c) fast_record(c, acc, e0, e1, Tr{}, Tr{});
+                    } else {
+#pragma unroll 2
+                        for (int c = np; c < nm; ++c) fast_record(c, acc, e0, e1, Tr{}, F{});
+                    }
                 }
             }
             if (wide || nm < n || GUARD) {
@@ -1458,11 +1467,11 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                     }
                 }
             }
-            sums[tid] += (double)fmaf(acc.x, edge_k[tid].x, acc_e.x);
-            sums[kConsumers + tid] += (double)fmaf(acc.y, edge_k[kConsumers + tid].x, acc_e.y);
             __syncwarp();
             if (lane == 0) mbar_arrive(b ? empty1 : empty0);
+            if (k % kFlush == kFlush - 1) flush();
         }
+        flush();
     }
     if (timeout && lane == 0) atomicOr(P.err, (int)KERR_WAIT_TIMEOUT);
 
