@@ -112,7 +112,7 @@ int32_t plan_batch(Ctx *c, const pstm_traces_desc *tr, const pstm_output_desc *o
         return fail(c, PSTM_ERR_UNSUPPORTED, "the batched form interpolates linearly");
     for (int i = 0; i < n_bins; ++i)
         if (bins[i].n_traces > 0)
-            bp.work.push_back({bins[i].trace_begin, bins[i].n_traces, bins[i].image, bins[i].fold});
+            bp.work.push_back({bins[i].trace_begin, bins[i].n_traces, bins[i].image, bins[i].fold, 1, 0});
     if (bp.work.empty()) return PSTM_OK;
     std::stable_sort(bp.work.begin(), bp.work.end(),
                      [](const BinWork &a, const BinWork &b) { return a.n_traces > b.n_traces; });
@@ -126,6 +126,11 @@ int32_t plan_batch(Ctx *c, const pstm_traces_desc *tr, const pstm_output_desc *o
     } else {
         auto it = c->tuned.find(class_key(tr, out, vel, prm));
         if (it != c->tuned.end()) P.max_chunk = it->second;
+    }
+    P.n_splits = 1;
+    for (BinWork &w : bp.work) {
+        w.shares = plan::split_traces((int64_t)P.n_pblk_x * P.n_pblk_y * P.n_tblk, w.n_traces);
+        P.n_splits = std::max(P.n_splits, w.shares);
     }
     bp.tt = prm->traveltime;
     bp.amp = tr->amp_dtype;

@@ -293,6 +293,8 @@ int32_t pstm_cuda_migrate_tile_runs_dev(void *ctx, const pstm_traces_desc *trace
         return cuda_fail(c, e, "writing the run list");
     tp.P.runs = reinterpret_cast<const int64_t *>(c->runs.ptr);
     tp.P.n_runs = (int32_t)rv.size();
+    tp.P.n_splits = plan::split_traces((int64_t)tp.P.n_pblk_x * tp.P.n_pblk_y * tp.P.n_tblk, tp.P.n_run_traces);
+    if (!plan::plan_grid(tp.P, 1, tp.L.grid)) return fail(c, PSTM_ERR_UNSUPPORTED, "tile too large for one launch");
     return launch_tile(c, tp);
 }
 

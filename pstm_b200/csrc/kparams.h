@@ -18,6 +18,8 @@ struct BinWork {
     int64_t n_traces;
     void *image;
     int32_t *fold;
+    int32_t shares;              // ranks among which its traces are divided (plan::split_traces)
+    int32_t pad;
 };
 
 // The scatter schedule: the panel cut into segments of seg_traces traces;
@@ -38,7 +40,7 @@ struct KParams {
     int32_t amp_kind;            // AmpKind
     int32_t pad0;
     const double *sx, *sy, *rx, *ry, *mx, *my, *w;   // w nullable
-    double dt_s, tstart_s;       // input sampling (seconds)
+    double dt_s, inv_dt, tstart_s;   // input sampling (seconds), 1 / dt
     float s_scale, s_offset;     // sample index s = T * s_scale + s_offset
     float s_guard_lo, s_guard_hi;  // fast-path accept window for s
     float s_rej_lo, s_rej_hi;    // outside [s_rej_lo, s_rej_hi] the pair is rejected

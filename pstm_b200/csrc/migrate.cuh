@@ -200,7 +200,7 @@ struct PtState {
     float t02v2, c1, e2;   // VTI: (t0/2)^2 v^2, 1+2eta, 2 eta / v^2
     float iv2r;            // 1/v_rms^2 (the curved+VTI ratio's hyperbolic leg; iv2 may be 1/v0^2)
     double v, eta;
-    double B;              // 1/(v dt)^2
+    double iv, B;          // 1/(v dt), its square
 };
 
 // The state of output point (p, t), evaluated in FP64 as
@@ -218,31 +218,32 @@ __device__ __forceinline__ void point_state(const KParams &P, int p, int t, int 
     double ap = v * t0 * 0.5 * P.tan_dip;
     if (ap < P.min_ap) ap = P.min_ap;
     else if (ap > P.max_ap) ap = P.max_ap;
+    const double rv = 1.0 / v, rvdt = rv * P.inv_dt;   // (divisions are what a small CTA's start waits for)
     s.v = v;
     s.eta = eta;
-    // seconds per unit of T
-    const double tu = unit == UNIT_METRES ? 1.0 / v : (unit == UNIT_SAMPLES ? P.dt_s : 1.0);
+    s.iv = rvdt;
+    // units of T per second
+    const double ut = unit == UNIT_METRES ? v : (unit == UNIT_SAMPLES ? P.inv_dt : 1.0);
     // the tests of T keep samples as their unit in metres too
-    const double tt = unit == UNIT_SECONDS ? 1.0 : P.dt_s;
+    const double tt = unit == UNIT_SECONDS ? 1.0 : P.inv_dt;
     // straight rays and VTI have T >= t0, so only t0 < 1.1 ms can give T <= 1 ms;
     // the curved-ray leg of the reference tends to 0 at large offsets
     const bool small_t = P.curved_kind || t0 < 0.0011;
     ts.t0h2 = (float)((t0 * 0.5) * (t0 * 0.5));
-    ts.tguard = (float)(0.001 / tt);
+    ts.tguard = (float)(0.001 * tt);
     ts.tg = small_t ? ts.tguard : -1.f;
-    const double th = t0 * 0.5 / P.dt_s;
+    const double th = t0 * 0.5 * P.inv_dt;
     ts.A = fmax(th * th, 1e-20);   // keeps the FP64 legs > 0 at t0 = 0
     ts.tzero = !(t0 > 0.0);
     ts.tz = ts.tzero && P.t0_zero_exact;
-    const double s0 = (0.0 - P.tstart_s) / P.dt_s;
+    const double s0 = (0.0 - P.tstart_s) * P.inv_dt;
     ts.tz_in = ts.tz && s0 >= 0.0 && s0 < (double)(P.ns - 1);
     ts.vz = ts.vz2 = ts.ivwc = 0.f;
     ts.vz64 = 0.0;
-    const float iv = (float)(1.0 / v);
-    float ivw = iv;
-    s.iv2 = (float)(1.0 / (v * v));
+    float ivw = (float)rv;
+    s.iv2 = (float)(rv * rv);
     s.iv2r = s.iv2;
-    s.B = 1.0 / (v * v * P.dt_s * P.dt_s);
+    s.B = rvdt * rvdt;
     if constexpr (TT == TT_CURVED || TT == TT_CURVED_VTI) {
         const double z = P.cr_k_zero ? P.cr_v0 * (t0 * 0.5) : (P.cr_v0 / P.cr_k) * (exp(P.cr_k * (t0 * 0.5)) - 1.0);
         ts.vz64 = P.cr_v0 + P.cr_k * z;
@@ -266,8 +267,8 @@ __device__ __forceinline__ void point_state(const KParams &P, int p, int t, int 
     s.aaA = P.aa_cA * ivw;
     s.aa_k = s.aaA * s.ivw_t;
     s.aa_thr = 0.01f * rcp_approx(unit == UNIT_SECONDS ? ivw : ivw * P.inv_dt_f);
-    s.thr_s = s.aa_thr * (float)(P.dt_s / tt);
-    const float Kt = P.obliquity ? (float)(t0 / tu) : 1.f;   // the obliquity's numerator
+    s.thr_s = unit == UNIT_SECONDS ? s.aa_thr * (float)P.dt_s : s.aa_thr;
+    const float Kt = P.obliquity ? (float)(t0 * ut) : 1.f;   // the obliquity's numerator
     s.K = P.spreading ? Kt * s.ivw_t : Kt;
     s.t02v2 = 0.f;
     s.c1 = 1.f;
@@ -291,8 +292,9 @@ __device__ __forceinline__ XState exact_state(const KParams &P, const TimeState 
     constexpr bool CURVED = TT == TT_CURVED || TT == TT_CURVED_VTI;
     XState x;
     x.A = ts.A;
-    x.C = ts.A / s.B * (CURVED ? (KZ ? 1.0 : P.cr_k2) : kQScale);
-    x.iv = 1.0 / (s.v * P.dt_s);
+    const double vdt = s.v * P.dt_s;
+    x.C = ts.A * vdt * vdt * (CURVED ? (KZ ? 1.0 : P.cr_k2) : kQScale);
+    x.iv = s.iv;
     x.c1 = 1.0 + 2.0 * s.eta;
     x.e2 = 2.0 * s.eta;
     x.vz = 2.0 * ts.vz64;
@@ -741,6 +743,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
     const int rank = (int)(blockIdx.x - item * splits);
     void *image = P.image;
     int64_t trace0 = 0, n_traces = P.runs ? P.n_run_traces : P.n_traces;
+    int shares = splits;   // ranks among which the item's traces are divided
     if (item >= n_items) {   // the fold-counting CTAs behind the items
         const int64_t k = (int64_t)blockIdx.x - n_items * splits;
         const int64_t out = k / P.n_pblk_fold;
@@ -762,6 +765,10 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
         trace0 = P.bins[b].trace0;
         n_traces = P.bins[b].n_traces;
         image = P.bins[b].image;
+        shares = P.bins[b].shares;
+        // a rank that a smaller bin has no use for leaves its slot at once (the
+        // cluster's barriers wait for the threads that have not exited)
+        if (rank >= shares) return;
     }
     // deep blocks first: their aperture is the widest; neighbours in y next to
     // each other, so that the CTAs that run together stage the same samples
@@ -821,7 +828,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                 unbounded |= !fine;
                 odd |= ts[g].tz;
                 ap_in = fminf(ap_in, st[g].ap * (1.f - P.taper_f));
-                const float th = (float)(P.ta[t] / 1000.0 / P.dt_s);
+                const float th = (float)(P.ta[t] * (0.001 * P.inv_dt));
                 t_lo = fminf(t_lo, th);
                 t_hi = fmaxf(t_hi, th);
                 apw = fmaxf(apw, st[g].ap);
@@ -888,16 +895,27 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
         double x0 = INFINITY, x1 = -INFINITY, y0 = INFINITY, y1 = -INFINITY;   // the patch's box
         float apmax = 0.f;
         HalfBounds hb[2];
-        for (int q = 0; q < P.px * P.py; ++q) {
-            const int jx = pbx * P.px + q / P.py, jy = pby * P.py + q % P.py;
-            if (jx >= P.nx || jy >= P.ny) continue;
-            const double x = P.xg ? P.xg[jx * P.ny + jy] : P.xa[jx], y = P.yg ? P.yg[jx * P.ny + jy] : P.ya[jy];
-            x0 = fmin(x0, x);
-            x1 = fmax(x1, x);
-            y0 = fmin(y0, y);
-            y1 = fmax(y1, y);
-            apmax = fmaxf(apmax, sh.apmax[q]);
+        if (lane < P.px * P.py) {
+            const int jx = pbx * P.px + lane / P.py, jy = pby * P.py + lane % P.py;
+            if (jx < P.nx && jy < P.ny) {
+                x0 = x1 = P.xg ? P.xg[jx * P.ny + jy] : P.xa[jx];
+                y0 = y1 = P.yg ? P.yg[jx * P.ny + jy] : P.ya[jy];
+                apmax = sh.apmax[lane];
+            }
         }
+#pragma unroll
+        for (int o = kPillars / 2; o > 0; o >>= 1) {
+            x0 = fmin(x0, __shfl_xor_sync(full, x0, o));
+            x1 = fmax(x1, __shfl_xor_sync(full, x1, o));
+            y0 = fmin(y0, __shfl_xor_sync(full, y0, o));
+            y1 = fmax(y1, __shfl_xor_sync(full, y1, o));
+            apmax = fmaxf(apmax, __shfl_xor_sync(full, apmax, o));
+        }
+        x0 = __shfl_sync(full, x0, 0);
+        x1 = __shfl_sync(full, x1, 0);
+        y0 = __shfl_sync(full, y0, 0);
+        y1 = __shfl_sync(full, y1, 0);
+        apmax = __shfl_sync(full, apmax, 0);
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
             hb[g] = {INFINITY, 0.f, INFINITY, 0.f, INFINITY, 0.f, INFINITY, 0.f};
@@ -920,7 +938,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
         const double reach = (double)apmax * (1.0 + 1e-6) + 1e-3;
         const double reach2 = reach * reach;
         // this rank's share of the traces, in whole chunks
-        const long long per = ((n_traces + splits - 1) / splits + kChunk - 1) / kChunk * kChunk;
+        const long long per = ((n_traces + shares - 1) / shares + kChunk - 1) / kChunk * kChunk;
         const long long v0 = min((long long)n_traces, rank * per), v1 = min((long long)n_traces, v0 + per);
         long long pos, end, left = 0;   // next trace, end of its range, (runs) traces of later ranges
         const long long stop = trace0 + v1;
@@ -1477,11 +1495,11 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
 
     // ---------------- epilogue: image += the sums (of every rank, in rank order)
     __syncthreads();
-    if (splits > 1) {
+    if (shares > 1) {
         cg::cluster_group cl = cg::this_cluster();
         cl.sync();
         if (rank == 0 && !producer) {
-            for (int r = 1; r < splits; ++r) {
+            for (int r = 1; r < shares; ++r) {
                 const double *other = cl.map_shared_rank(sums, r);
                 sums[tid] += other[tid];
                 sums[kConsumers + tid] += other[kConsumers + tid];

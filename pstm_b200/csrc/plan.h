@@ -63,6 +63,30 @@ inline int32_t check_args(const pstm_traces_desc *tr, const pstm_output_desc *ou
     return PSTM_OK;
 }
 
+// CTAs of a cluster that share the traces of an item.  A CTA's start -- its
+// points' state, the first selection and copies -- costs about kStartChunks chunks
+// of traces, and 2 x 148 CTAs run at a time, so S CTAs per item take about
+// ceil(items S / 296) (kStartChunks + chunks / S).  A cluster also starts and ends
+// together, which cost 14 % on a 32 x 32 x 800 tile (1664 items, 625 chunks) that
+// this count has gain 2 % from S = 4; so every doubling has to win 15 %.  By the
+// tile's size and the output's own traces alone, so that
+// a bin and the same traces as a tile of their own are summed in the same order.
+constexpr int kStartChunks = 4;
+inline int split_traces(int64_t items, int64_t n_traces) {
+    int best = 1;
+    double least = INFINITY;
+    for (int s = 1; s <= kMaxSplits; s *= 2) {
+        const int64_t waves = (items * s + 295) / 296;
+        const int64_t chunks = (n_traces + (int64_t)kChunk * s - 1) / ((int64_t)kChunk * s);
+        const double cost = (double)waves * (double)(kStartChunks + chunks);
+        if (cost < 0.85 * least) {
+            least = cost;
+            best = s;
+        }
+    }
+    return best;
+}
+
 inline KParams make_params(const pstm_traces_desc *tr, const pstm_output_desc *out, const pstm_velocity_desc *vel,
                     const pstm_params *prm) {
     KParams P;
@@ -81,6 +105,7 @@ inline KParams make_params(const pstm_traces_desc *tr, const pstm_output_desc *o
     P.mx = tr->midpoint_x; P.my = tr->midpoint_y;
     P.w = tr->weights;
     P.dt_s = tr->sample_rate_ms / 1000.0;
+    P.inv_dt = 1.0 / P.dt_s;
     P.tstart_s = tr->start_time_ms / 1000.0;
     P.s_scale = (float)(1.0 / P.dt_s);
     P.s_offset = (float)(-P.tstart_s / P.dt_s);
@@ -165,11 +190,7 @@ inline KParams make_params(const pstm_traces_desc *tr, const pstm_output_desc *o
     P.n_tblk = (out->nt + kTimes - 1) / kTimes;
     P.n_pblk_fold = (int32_t)(((int64_t)out->nx * out->ny + kFoldPillars - 1) / kFoldPillars);
     P.max_chunk = kChunk;
-    // CTAs that share an item's traces: enough for two per SM four times over
-    // (148 SMs), by the tile's size alone, so that a bin and the same traces as
-    // a tile of their own are summed in the same order.
-    P.n_splits = 1;
-    while (P.n_splits < kMaxSplits && best * P.n_tblk * P.n_splits < 4 * 2 * 148) P.n_splits *= 2;
+    P.n_splits = split_traces(best * P.n_tblk, tr->n_traces);
     return P;
 }
 
