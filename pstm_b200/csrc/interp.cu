@@ -43,6 +43,17 @@ constexpr int kInterpThreads = 128;
 #define PSTM_INTERP_MIN_CTAS 8
 #endif
 
+// sqrt(q) for q > 0 from the hardware's approximate reciprocal square root h and one
+// third-order step: w = q h, r = 1 - w h, w (1 + r / 2 + 3 r^2 / 8).  Full FP64, where
+// Newton's step would leave 2^-40 in the sample index of an FP64 image.
+__device__ __forceinline__ double sqrt_third(double q) {
+    double h;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(h) : "d"(q));
+    const double w = q * h;
+    const double r = fma(-w, h, 1.0);
+    return fma(w * r, fma(r, 0.375, 0.5), w);
+}
+
 template <int AMP, typename R = double>
 __device__ inline R sample_at(const unsigned char *row, int64_t i) {
     return (R)amp_at<AMP>(row, (int)i);
@@ -106,11 +117,12 @@ __device__ __forceinline__ R taylor_from(R u) {
     if constexpr (N + 2 > LAST) return (R)taylor<N>;
     else return taylor_from<N + 2, LAST, R>(u) * u + (R)taylor<N>;
 }
-// Last power of y = pi f / HW that matters: the next one's term is below 2^-54.
+// Last power of y that matters: the next ones' terms are below 2^-46 (the sample
+// index's Newton step leaves 2^-40).
 constexpr int taylor_last(double y) {
     int n = 1;
     double t = y;
-    while (t > 0x1p-54) t *= y / ++n;
+    while (t > 0x1p-46) t *= y / ++n;
     return n;
 }
 
@@ -142,31 +154,49 @@ struct Wide {
     const unsigned char *row;
     int i, i_max;
     R f, C, S, acc, norm;
-    R E[HW];   // E[k - 1]: product of the D's but D_k
+    R E[HW], FE[HW];   // E[k - 1]: product of the D's but D_k; f E
 
-    template <int K>
-    __device__ __forceinline__ void tap(bool live) {
-        const R sg = (K & 1) ? R(-1) : R(1);
-        const R e = E[K > 0 ? K - 1 : -K] * (f - (R)(1 - K));   // x_{1-K} E
-        R w;
+    // C cos + S sin with compile-time factors; 0 and 1 cost nothing
+    static __device__ __forceinline__ R rotate(R a, R b, double ca, double sb) {
+        if (ca == 0.0) return sb == 1.0 ? b : (sb == -1.0 ? -b : b * (R)sb);
+        if (sb == 0.0) return ca == 1.0 ? a : (ca == -1.0 ? -a : a * (R)ca);
+        return a * (R)ca + b * (R)sb;
+    }
+    // taps J and J - HW, whose window angles differ by pi: the Hann window's cosine
+    // (and the Lanczos sine) changes its sign from one to the other
+    template <int J>
+    __device__ __forceinline__ void tap_pair(bool live) {
         if constexpr (LANCZOS) {
-            const R sn = S * (R)win_cos<HW, K> - C * (R)win_sin<HW, K>;
-            w = sg * sn * e * e;
+            const R sn = rotate(S, C, win_cos<HW, J>, -win_sin<HW, J>);
+            const R ea = x_over<J>(), eb = x_over<J - HW>();
+            const R wa = (J & 1 ? -sn : sn) * ea * ea, wb = ((J - HW) & 1 ? sn : -sn) * eb * eb;
+            add(wa, i + J);
+            add(wb, i + J - HW);
         } else {
-            const R cs = C * (R)win_cos<HW, K> + S * (R)win_sin<HW, K>;
-            w = (sg + sg * cs) * e;
+            const R cs = rotate(C, S, win_cos<HW, J>, win_sin<HW, J>);
+            R wa = (J & 1 ? R(-1) - cs : R(1) + cs) * x_over<J>();
+            const R wb = (J & 1 ? cs - R(1) : R(1) - cs) * x_over<J - HW>();
+            int ja = i + J;
+            if constexpr (J == HW) {   // beyond the window (and possibly the trace) for f < 0
+                wa = live ? wa : R(0);
+                ja = min(ja, i_max);
+            }
+            add(wa, ja);
+            add(wb, i + J - HW);
         }
-        int j = i + K;
-        if constexpr (K == HW && !LANCZOS) {   // beyond the window (and possibly the trace) for f < 0
-            w = live ? w : R(0);
-            j = min(j, i_max);
-        }
+    }
+    template <int K>   // E / x_K = x_{1-K} E_k
+    __device__ __forceinline__ R x_over() const {
+        constexpr int k = K > 0 ? K : 1 - K;
+        return FE[k - 1] + (R)(K - 1) * E[k - 1];
+    }
+    __device__ __forceinline__ void add(R w, int j) {
         acc += sample_at<AMP, R>(row, j) * w;
         norm += w;
     }
-    template <int... K>
-    __device__ __forceinline__ void taps(std::integer_sequence<int, K...>, bool live) {
-        (tap<K - HW + 1>(live), ...);
+    template <int... J>
+    __device__ __forceinline__ void taps(std::integer_sequence<int, J...>, bool live) {
+        (tap_pair<J + 1>(live), ...);
     }
     __device__ __forceinline__ R run(const unsigned char *r, int ns, int i0, R f0) {
         if (i0 < HW || i0 >= ns - HW) return sample_at<AMP, R>(r, i0) * (R(1) - f0) + sample_at<AMP, R>(r, i0 + 1) * f0;
@@ -200,12 +230,21 @@ struct Wide {
         for (int k = HW - 1; k >= 0; --k) {
             E[k] *= suf;
             suf *= D[k];
+            FE[k] = f * E[k];
         }
         acc = norm = R(0);
-        taps(std::make_integer_sequence<int, 2 * HW>{}, f >= R(0));
+        taps(std::make_integer_sequence<int, HW>{}, f >= R(0));
         return norm != R(0) ? acc * rcp_r(norm) : R(0);
     }
 };
+
+// 0.5 (1 + cos(pi x)) = cos^2(pi x / 2), 0 <= x <= 1, from cos's Taylor polynomial.
+template <typename R>
+__device__ __forceinline__ R taper_weight_r(R x) {
+    const R y = x * (R)(0.5 * kPi);
+    const R c = taylor_from<0, taylor_last(0.5 * kPi), R>(y * y);
+    return c * c;
+}
 
 template <int TT>
 __device__ inline double tt_of(double t0, double ds2, double dr2, double v, double eta, double v0, double k) {
@@ -215,7 +254,7 @@ __device__ inline double tt_of(double t0, double ds2, double dr2, double v, doub
 // Per-trace values a warp stages in shared memory for the CTA's pillar.
 struct Staged {
     double ds2[32], dr2[32], d[32], w[32], m[32];
-    int tr[32];
+    const unsigned char *row[32];
 };
 
 // R: double on the exact path (FP64 end to end); float on the fast path,
@@ -242,11 +281,20 @@ __global__ void __launch_bounds__(kInterpThreads, PSTM_INTERP_MIN_CTAS) migrate_
         const double z = P.cr_k_zero ? P.cr_v0 * (t0 * 0.5) : (P.cr_v0 / P.cr_k) * (exp(P.cr_k * (t0 * 0.5)) - 1.0);
         vw = P.cr_v0 + P.cr_k * z;
     }
-    const double gmax = P.aa_gmax, fdom = P.aa_fdom;
-    const double inv_vw = 1.0 / vw;
     const double taper_start = ap * (1.0 - P.taper);
     const double inv_taper_w = ap > taper_start ? 1.0 / (ap - taper_start) : 0.0;
-    const double iv2 = 1.0 / (v * v), t0h2 = (t0 * 0.5) * (t0 * 0.5), inv_dt = 1.0 / P.dt_s;
+    const double inv_dt = 1.0 / P.dt_s, s_off = -P.tstart_s * inv_dt;
+    // The weights need L = v_w T alone: spreading 1 / L, obliquity (t0 v_w) / L,
+    // sin(theta) = m / L.  On straight rays L is the sum of the legs' sqrt(C + h^2), C =
+    // (t0 v / 2)^2, and the sample index follows from it.
+    const double C = 0.25 * t0 * t0 * v * v, iv = inv_dt / v;
+    const R K = P.obliquity ? (R)(t0 * vw) : R(1);
+    const int n_inv = (P.spreading ? 1 : 0) + (P.obliquity ? 1 : 0);
+    const R aa_A = (R)(4.0 * P.aa_gmax * P.aa_fdom / vw);
+    const R aa_lo = fmax(R(0), R(1) - aa_A), aa_hi = fmax(R(0), (R)(1.0 - P.aa_fdom / 500.0));
+    // T <= 1 ms, where the weights do not apply, needs t0 < 1.1 ms or curved rays
+    const bool small_t = P.curved_kind || t0 < 0.0011;
+    const double L2_min = small_t ? 0.002 * vw : -1.0;
 
     Staged &S = S_all[warp];
     // Largest aperture over the warp's output times: a trace farther than it
@@ -280,26 +328,30 @@ __global__ void __launch_bounds__(kInterpThreads, PSTM_INTERP_MIN_CTAS) migrate_
             S.d[j] = d;
             S.w[j] = P.w ? P.w[tr] : 1.0;
             S.m[j] = fmax(fabs(dxm), fabs(dym));
-            S.tr[j] = (int)tr;
+            S.row[j] = reinterpret_cast<const unsigned char *>(P.amps) + tr * P.amp_stride * (int64_t)P.elem;
         }
         __syncwarp();
         for (int j = 0; j < n_kept; ++j) {
             const double dj = S.d[j];
             if (!tv || dj > ap) continue;
             const double ds2 = S.ds2[j], dr2 = S.dr2[j];
-            double T;
-            switch (tt) {
-            case TT_CURVED: T = tt_of<TT_CURVED>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
-            case TT_VTI: T = tt_of<TT_VTI>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
-            case TT_CURVED_VTI: T = tt_of<TT_CURVED_VTI>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
-            default:   // the straight legs with this thread's 1/v^2 and the Newton-refined sqrt
-                T = sqrt_newton(fma(ds2, iv2, t0h2)) + sqrt_newton(fma(dr2, iv2, t0h2));
-                break;
+            double s, L2;   // sample index, 2 v_w T
+            if (tt == TT_STRAIGHT) {
+                L2 = sqrt_third(fmax(ds2 + C, 1e-12)) + sqrt_third(fmax(dr2 + C, 1e-12));
+                s = fma(L2, iv, s_off);
+                L2 += L2;
+            } else {
+                double T;
+                switch (tt) {
+                case TT_CURVED: T = tt_of<TT_CURVED>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
+                case TT_VTI: T = tt_of<TT_VTI>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
+                default: T = tt_of<TT_CURVED_VTI>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
+                }
+                s = (T - P.tstart_s) * inv_dt;
+                L2 = 2.0 * vw * T;
             }
-            const double s = (T - P.tstart_s) * inv_dt;
             if (!(s >= 0.0 && s < (double)(P.ns - 1))) continue;
-            const unsigned char *row =
-                reinterpret_cast<const unsigned char *>(P.amps) + ((int64_t)S.tr[j] * P.amp_stride) * (int64_t)P.elem;
+            const unsigned char *row = S.row[j];
             // integer and fraction without conversions: s + 1.5 2^52 has the nearest
             // integer in its low word
             const double near = s + 6755399441055744.0;
@@ -313,26 +365,20 @@ __global__ void __launch_bounds__(kInterpThreads, PSTM_INTERP_MIN_CTAS) migrate_
             if constexpr (HW > 0) amp = Wide<AMP, HW, LANCZOS, R>().run(row, P.ns, i0, (R)fr);
             else amp = interpolate_narrow<AMP, R>(row, P.ns, i0, (R)fr, method);
             R w = (R)S.w[j];
-            if (dj > taper_start) {
-                const R x = (R)((dj - taper_start) * inv_taper_w);
-                R cw;
-                if constexpr (sizeof(R) == 8) cw = cospi(x);
-                else cw = cospif(x);
-                w *= R(0.5) * (R(1) + cw);
+            if (dj > taper_start) w *= taper_weight_r((R)((dj - taper_start) * inv_taper_w));
+            const R inv = R(2) * rcp_r((R)L2);
+            R g = R(1);
+            if (n_inv == 2) g = K * inv * inv;
+            else if (n_inv == 1) g = K * inv;
+            g = L2 > L2_min ? g : R(1);
+            if (P.aa && L2 >= L2_min) {
+                const R sn = (R)S.m[j] * inv;
+                R y = R(1) - aa_A * sn;
+                y = y > aa_hi ? aa_hi : y;
+                y = y < aa_lo ? aa_lo : y;
+                g = sn >= R(0.01) ? g * y : g;
             }
-            // One reciprocal of T per pair and 1/v per thread serve the AA,
-            // spreading and obliquity terms: sin = m / (v T), f_max = min(v /
-            // (4 gmax sin), 500 Hz) so f_dom / f_max = f_dom max(4 gmax sin / v,
-            // 1 / 500), spreading 1 / (v T), obliquity t0 / T.
-            const R Tr = (R)T, inv_T = rcp_r(Tr), ivw = (R)inv_vw;
-            if (P.aa && T >= 0.001) {
-                const R st = fmin((R)S.m[j] * inv_T * ivw, R(1));
-                if (st >= R(0.01))
-                    w *= fmax(R(0), R(1) - (R)fdom * fmax(R(4) * (R)gmax * st * ivw, R(1) / R(500)));
-            }
-            if (P.spreading && T > 0.001) w *= inv_T * ivw;
-            if (P.obliquity && T > 0.001) w *= (R)t0 * inv_T;
-            acc += (double)(amp * w);
+            acc += (double)(amp * (w * g));
         }
         __syncwarp();   // the next batch overwrites the staged values
     }
