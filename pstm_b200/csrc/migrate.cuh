@@ -14,9 +14,9 @@
 //             distances, rounded once) in three classes: PLAIN, where every
 //             test of the pair loop is known to pass for every lane; MID, where
 //             only the aperture's taper and the trace ends are open; and EDGE,
-//             the rest.  Then they
-//             run the classes' pair loops; every four chunks their FP32 sums
-//             go into FP64.  16-bit samples are first widened to FP32 in shared memory.
+//             the rest.  Then they run the classes' pair loops; every four
+//             chunks their FP32 sums go into FP64.  16-bit samples are first
+//             widened to FP32 in shared memory.
 // No warp waits for another consumer (except to widen), so uneven chunks and the
 // producer's memory latency are hidden; the first form, in which the eight warps
 // selected, staged and built in turn between CTA barriers, lost 12 % of its warp
@@ -27,8 +27,16 @@
 // so results do not depend on scheduling.  The image is added into once, in the
 // epilogue.  Further CTAs of the same launch count the fold.
 //
-// What bounds it: instruction issue, then the MUFU pipe (two FP64 reciprocal
-// square roots and one reciprocal per straight pair: 24 of its cycles).
+// What bounds it: issue.  Dispatch costs of one warp add up (measured, cycles per
+// SM sub-partition: FP64 2.1, or 3.4 with three register operands; FP32 1.15,
+// packed FP32 2.3; shared-memory reads, MUFU and integer about 1), and a PLAIN
+// straight-ray pair with AA is 20 of FP64, 9 of FP32, 5 integer, 3 MUFU, 3 reads and
+// 2 moves: 43 cycles, which is what it takes (39 without AA, 54-70 MID), while its
+// three MUFU operations occupy that pipe for 24.  Unrolling by 1 to 4, software
+// pipelining, scalar instead of packed FP32, and one or three CTAs per SM instead
+// of two are all within 8 % of each other or slower.  Records cost 220 cycles a warp
+// and chunk.  64 x 64 pillars x 1500 times x 16,384 traces, 3-D velocity, AA: 191 ms
+// with whole rows staged and state reloaded from tables per chunk, 118 ms now.
 //
 // Reference semantics (paths relative to the reference project):
 //   loop structure, fold, aperture, taper, weights  numba_cpu_optimized.py:147-231
@@ -821,7 +829,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
             point_state<TT>(P, p, valid ? t : P.nt - 1, UNIT, ts[g], st[g]);
             if (EXACT) xs[g] = exact_state<TT, KZ>(P, ts[g], st[g]);
             const float A = (float)ts[g].A, B = (float)st[g].B, e = (float)st[g].eta, vz = ts[g].vz;
-            bool fine = A < 1e30f && B > 0.f && B < 1e30f;
+            bool fine = A < 1e30f && B > 0.f && B < 1e30f && st[g].iv > 0.0;   // (also not NaN)
             if (TT == TT_VTI || TT == TT_CURVED_VTI) fine = fine && e >= -0.15f && e < 1e3f;
             if (CURVED) fine = fine && vz > 0.f && vz < 1e15f;
             if (valid) {
