@@ -43,17 +43,6 @@ constexpr int kInterpThreads = 128;
 #define PSTM_INTERP_MIN_CTAS 8
 #endif
 
-// sqrt(q) for q > 0 from the hardware's approximate reciprocal square root h and one
-// third-order step: w = q h, r = 1 - w h, w (1 + r / 2 + 3 r^2 / 8).  Full FP64, where
-// Newton's step would leave 2^-40 in the sample index of an FP64 image.
-__device__ __forceinline__ double sqrt_third(double q) {
-    double h;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(h) : "d"(q));
-    const double w = q * h;
-    const double r = fma(-w, h, 1.0);
-    return fma(w * r, fma(r, 0.375, 0.5), w);
-}
-
 template <int AMP, typename R = double>
 __device__ inline R sample_at(const unsigned char *row, int64_t i) {
     return (R)amp_at<AMP>(row, (int)i);
@@ -283,11 +272,16 @@ __global__ void __launch_bounds__(kInterpThreads, PSTM_INTERP_MIN_CTAS) migrate_
     }
     const double taper_start = ap * (1.0 - P.taper);
     const double inv_taper_w = ap > taper_start ? 1.0 / (ap - taper_start) : 0.0;
-    const double inv_dt = 1.0 / P.dt_s, s_off = -P.tstart_s * inv_dt;
+    const double inv_dt = 1.0 / P.dt_s;
     // The weights need L = v_w T alone: spreading 1 / L, obliquity (t0 v_w) / L,
-    // sin(theta) = m / L.  On straight rays L is the sum of the legs' sqrt(C + h^2), C =
-    // (t0 v / 2)^2, and the sample index follows from it.
-    const double C = 0.25 * t0 * t0 * v * v, iv = inv_dt / v;
+    // sin(theta) = m / L.  The sample index is formed in seconds with one Newton step:
+    // a windowed sinc jumps by 0.4 % of a sample where its nearest sample changes, so
+    // another rounding of the index (in metres, or a third-order step; neither faster: 32.1
+    // against 31.8-32.1 ms for 40 x 40 x 500 points and 6,000 traces) moves a
+    // few pairs of 10^9 across a jump and an FP64 image by 2e-9.
+    const double iv2 = 1.0 / (v * v);
+    // (at t0 = 0 above 0, so that a leg of length 0 has a root)
+    const double t0h2 = fmax((t0 * 0.5) * (t0 * 0.5), 1e-30), vw2 = 2.0 * vw;
     const R K = P.obliquity ? (R)(t0 * vw) : R(1);
     const int n_inv = (P.spreading ? 1 : 0) + (P.obliquity ? 1 : 0);
     const R aa_A = (R)(4.0 * P.aa_gmax * P.aa_fdom / vw);
@@ -335,21 +329,14 @@ __global__ void __launch_bounds__(kInterpThreads, PSTM_INTERP_MIN_CTAS) migrate_
             const double dj = S.d[j];
             if (!tv || dj > ap) continue;
             const double ds2 = S.ds2[j], dr2 = S.dr2[j];
-            double s, L2;   // sample index, 2 v_w T
-            if (tt == TT_STRAIGHT) {
-                L2 = sqrt_third(fmax(ds2 + C, 1e-12)) + sqrt_third(fmax(dr2 + C, 1e-12));
-                s = fma(L2, iv, s_off);
-                L2 += L2;
-            } else {
-                double T;
-                switch (tt) {
-                case TT_CURVED: T = tt_of<TT_CURVED>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
-                case TT_VTI: T = tt_of<TT_VTI>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
-                default: T = tt_of<TT_CURVED_VTI>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
-                }
-                s = (T - P.tstart_s) * inv_dt;
-                L2 = 2.0 * vw * T;
+            double T;
+            switch (tt) {
+            case TT_CURVED: T = tt_of<TT_CURVED>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
+            case TT_VTI: T = tt_of<TT_VTI>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
+            case TT_CURVED_VTI: T = tt_of<TT_CURVED_VTI>(t0, ds2, dr2, v, eta, P.cr_v0, P.cr_k); break;
+            default: T = sqrt_newton(fma(ds2, iv2, t0h2)) + sqrt_newton(fma(dr2, iv2, t0h2)); break;
             }
+            const double s = (T - P.tstart_s) * inv_dt, L2 = vw2 * T;
             if (!(s >= 0.0 && s < (double)(P.ns - 1))) continue;
             const unsigned char *row = S.row[j];
             // integer and fraction without conversions: s + 1.5 2^52 has the nearest
