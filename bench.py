@@ -431,8 +431,8 @@ def accuracy_vs_fp64(kernel_factory, sv, cfg, n_tr, amps_host, pillars=2):
 def measure_forms(args, k_plain, tb, amps, tile_args, my_tiles, pairs_per_step, world, dist, sv, cfg):
     """Plain form (exact sample index, FP32 traces) and the precision form (FP16
     traces with a power-of-two scale per trace carried by the trace weight,
-    FP32 traveltime, sample index and trace-end tests, compensated FP32
-    accumulation; the FP32-arithmetic kernel on FP32 traces, FP16 with the
+    FP32 traveltime, sample index and trace-end tests, FP64 sums of short
+    FP32 partial sums; the FP32-arithmetic kernel on FP32 traces, FP16 with the
     FP64 sample index or with FP64 trace-end re-decisions, and BF16 beside
     it): pairs/s on the timed tiles of the full case-2 panel and rel-L2 vs
     the FP64 oracle on the FP32 traces."""

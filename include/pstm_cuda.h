@@ -123,7 +123,7 @@ typedef struct {
     double curved_v0, curved_k;   /* V(z) = v0 + k z */
     const double *eta;            /* nullable: eta_constant; else (nt) or (nx, ny, nt) */
     int32_t eta_is_3d;
-    int32_t compensated;          /* 1: compensated (TwoSum) FP32 accumulation */
+    int32_t compensated;          /* 1: FP32 partial sums over one chunk (<= 32 traces), 0: over four; then FP64 */
     double eta_constant;
     int32_t precision;            /* pstm_precision */
     int32_t interpolation;        /* pstm_interp; KernelConfig.interpolation_method, base.py:213 */

@@ -69,7 +69,7 @@ struct KParams {
     int32_t fold3d;
     int32_t nx, ny, nt;
     int32_t px, py;              // pillar patch of one CTA (px * py pillars)
-    int32_t pad2;
+    int32_t flush_mask;          // FP32 sums go into FP64 after chunks k with k & mask == mask
     const double *xa, *ya, *xg, *yg, *ta;   // xg/yg nullable
 
     // ---- velocity ----

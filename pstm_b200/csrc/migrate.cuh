@@ -14,7 +14,7 @@
 //             distances, rounded once) in three classes: PLAIN, where every
 //             test of the pair loop is known to pass for every lane; MID, where
 //             only the aperture's taper and the trace ends are open; and EDGE,
-//             the rest.  Then they run the classes' pair loops; every four
+//             the rest.  Then they run the classes' pair loops; every four (or one)
 //             chunks their FP32 sums go into FP64.  16-bit samples are first
 //             widened to FP32 in shared memory.
 // No warp waits for another consumer (except to widen), so uneven chunks and the
@@ -71,7 +71,7 @@ constexpr int kChunk = 32;                  // traces per chunk, upper bound: on
 constexpr int kRowPitch = 256;              // staged samples per trace with 32 traces per chunk
 constexpr int kPool = kChunk * kRowPitch;   // staged samples of one buffer
 constexpr int kMaxSplits = 8;               // CTAs of a cluster that share an item's traces
-constexpr int kFlush = 4;                   // chunks whose FP32 sums are added into FP64 together
+constexpr int kFlush = 4;                   // chunks whose FP32 sums are added into FP64 together (a power of 2)
 constexpr int kFoldPillars = 8;             // pillars per fold-counting CTA
 constexpr int kWaitIters = 1 << 20;         // default bound of every mbarrier wait loop (KParams::wait_iters)
 
@@ -1495,7 +1495,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(b ? empty1 : empty0);
-            if (k % kFlush == kFlush - 1) flush();
+            if ((k & P.flush_mask) == P.flush_mask) flush();
         }
         flush();
     }

@@ -96,9 +96,9 @@ class CudaKernel:
         power-of-two scale per trace carried by the trace weight
         (:meth:`to_f16_panel`, which also converts device panels).
     compensated:
-        TwoSum-compensated FP32 partial sums between the flushes into the
-        image (``True``/``False``); ``"auto"`` compensates for 16-bit traces
-        (the precision form) and not for FP32 traces.
+        FP32 partial sums go into FP64 sums after at most 32 traces (``True``)
+        or 128 (``False``); ``"auto"`` is ``True`` for 16-bit traces (the
+        precision form) and ``False`` for FP32 traces.
     velocity_mode:
         ``"exact"`` uses a 3-D velocity slice per pillar; ``"auto"`` follows the
         Metal host rule (``metal_compiled.py:631-664``): the centre pillar is
@@ -335,8 +335,8 @@ class CudaKernel:
         return p
 
     def _auto_compensation(self, prm, td) -> None:
-        """compensated="auto": TwoSum-compensated partial sums for 16-bit traces
-        (the precision form), plain FP32 partials for FP32 traces."""
+        """compensated="auto": FP64 sums of short FP32 partial sums for 16-bit
+        traces (the precision form), of longer ones for FP32 traces."""
         if self._compensated == "auto":
             prm.compensated = int(td.amp_dtype != nat.AMP_F32)
 
