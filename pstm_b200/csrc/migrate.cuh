@@ -1156,7 +1156,10 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                 word = (unsigned)__double2hiint(v);
                 f = __uint_as_float(__funnelshift_r((unsigned)__double2loint(v), 0x7Fu, 9));
                 T = scaled_double_to_float(T2);
-                if constexpr (decltype(clamp_c)::value) T_test = CURVED ? T : scaled_double_to_float(T2 * xs[g].iv);
+                if constexpr (decltype(clamp_c)::value) {   // (nearest but for straight rays: these only truncate)
+                    if constexpr (TT == TT_STRAIGHT) T_test = scaled_double_to_float(T2 * xs[g].iv);
+                    else T_test = (float)((CURVED ? T2 : T2 * xs[g].iv) * (1.0 / kTimeScale));
+                }
             } else {
                 const float4 B = *reinterpret_cast<const float4 *>(r);
                 float4 Cf = make_float4(0.f, 0.f, 0.f, 0.f);
