@@ -309,8 +309,8 @@ __device__ __forceinline__ XState exact_state(const KParams &P, const TimeState 
     x.vz2 = ts.vz64 * ts.vz64;
     return x;
 }
-// The squared distances h^2 of an EXACT record: straight and VTI carry them times
-// kQScale, the curved kinds times k^2.
+// The squared distances h^2 of an EXACT record (finite: the producer drops other
+// traces): straight and VTI carry them times kQScale, the curved kinds times k^2.
 template <int TT, bool KZ>
 __device__ __forceinline__ double record_square(const KParams &P, double x) {
     if constexpr (TT == TT_CURVED || TT == TT_CURVED_VTI) return KZ ? x : P.cr_k2 * x;
@@ -1048,6 +1048,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                 if (P.w) w = P.w[id];
             }
             float lo = INFINITY, hi = -INFINITY;
+            bool finite;
             {
                 auto near2 = [&](double x, double y) {
                     const float a = (float)fmax(fmax(x0 - x, x - x1), 0.0), b = (float)fmax(fmax(y0 - y, y - y1), 0.0);
@@ -1058,6 +1059,10 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                     return (a * a + b * b) * (1.f + 1e-6f);
                 };
                 const float s0 = near2(sx, sy), s1 = far2(sx, sy), r0 = near2(rx, ry), r1 = far2(rx, ry);
+                // A coordinate that is not finite, or farther than 1.8e19 m: the trace has no sample
+                // for any pair.  Asked here, because the bounds' fminf and fmaxf lose a NaN, and a
+                // trace that they wrongly call PLAIN is read without a test of its index.
+                finite = s1 < INFINITY && r1 < INFINITY;
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
                     if (hb[g].A0 == INFINITY) continue;   // no live time in this half
@@ -1072,7 +1077,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
             const float s_hi = hi * (1.f + 2e-6f) - start_s + margin;
             const bool none = lo == INFINITY && hi == -INFINITY;      // only T = 0 times
             const bool known = !any_unbounded && s_lo <= s_hi;        // (not NaN)
-            int flags = (!any_unbounded && none) || (known && (s_hi < 0.f || s_lo >= last)) ? TRACE_DROP : 0;
+            int flags = !finite || (!any_unbounded && none) || (known && (s_hi < 0.f || s_lo >= last)) ? TRACE_DROP : 0;
             if (known && lo > t_min && fabs(w) < 1e30) flags |= TRACE_SURE;
             if (known && s_lo >= 0.f && s_hi < last) flags |= TRACE_INSIDE;
             int a = 0, e = P.ns - 1;   // samples the pairs can read
