@@ -923,7 +923,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
         x1 = __shfl_sync(full, x1, 0);
         y0 = __shfl_sync(full, y0, 0);
         y1 = __shfl_sync(full, y1, 0);
-        apmax = __shfl_sync(full, apmax, 0);
+        apmax = fminf(__shfl_sync(full, apmax, 0), (float)P.max_ap);
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
             hb[g] = {INFINITY, 0.f, INFINITY, 0.f, INFINITY, 0.f, INFINITY, 0.f};
@@ -1362,7 +1362,8 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                 // the FP64 sqrt is needed only where the aperture cut is hard
                 d = hard_cut ? (float)sqrt(d2) : sqrt_approx((float)d2);
                 row = tab.row[lane];
-                if (d <= sh.warp[warp].apw) {
+                // the maximum aperture cuts for itself: a minimum above it raises every time's own
+                if (d <= sh.warp[warp].apw && d2 <= P.fold_d2_max) {
                     const double dxs = ox - tab.sx[lane], dys = oy - tab.sy[lane];
                     const double dxr = ox - tab.rx[lane], dyr = oy - tab.ry[lane];
                     ds2 = dxs * dxs + dys * dys;
