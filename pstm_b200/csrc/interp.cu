@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(kInterpThreads, PSTM_INTERP_MIN_CTAS) migrate_
             const double d2 = dxm * dxm + dym * dym;
             in_fold = d2 <= P.fold_d2_max;
             d = sqrt(d2);
-            keep = !(d > ap_w);
+            keep = in_fold && !(d > ap_w);   // the maximum cuts for itself, also below the minimum
         }
         const unsigned kb = __ballot_sync(0xffffffffu, keep);
         cnt += __popc(__ballot_sync(0xffffffffu, in_fold));

@@ -98,3 +98,13 @@ def test_every_form_cuts_at_the_maximum(form, cuda_kernel_factory):
     got = dataclasses.replace(got, image=got.image.cpu().numpy(), fold=got.fold.cpu().numpy())
     torch.cuda.synchronize()
     _check(tb, vel, cfg, "straight_ray", "exact", got, ref)
+
+
+@pytest.mark.parametrize("precision", ["exact", "fast"])
+@pytest.mark.parametrize("method", ["nearest", "cubic", "sinc8", "lanczos3"])
+def test_interpolators_cut_at_the_maximum(method, precision, cuda_kernel_factory):
+    tb, vel, cfg = _case(max_aperture_m=300.0, min_aperture_m=500.0, interpolation_method=method)
+    k = cuda_kernel_factory(cfg, precision=precision)
+    got, ref = _out(), _out()
+    k.migrate_tile(tb, got, vel)
+    _check(tb, vel, cfg, "straight_ray", precision, got, ref)
