@@ -365,7 +365,8 @@ __global__ void __launch_bounds__(256) probe_kernel(const __grid_constant__ KPar
         PtState s;
         point_state<TT_STRAIGHT>(P, p, t, UNIT_SECONDS, ts, s);
         const double dxm = ox - P.mx[tr], dym = oy - P.my[tr];
-        const bool act = (float)sqrt(dxm * dxm + dym * dym) <= s.ap;
+        const double d2 = dxm * dxm + dym * dym;
+        const bool act = d2 <= P.fold_d2_max && (float)sqrt(d2) <= s.ap;
         const float dxs = (float)(ox - P.sx[tr]), dys = (float)(oy - P.sy[tr]);
         const float dxr = (float)(ox - P.rx[tr]), dyr = (float)(oy - P.ry[tr]);
         const float r[7] = {(float)(P.ta[t] / 1000.0), dxs, dys, dxr, dyr, 1.f / (float)(1.0 / s.v), (float)s.eta};
@@ -413,9 +414,10 @@ __global__ void __launch_bounds__(128) migrate_learned_kernel(const KParams P, c
     for (int64_t tr = 0; tr < P.n_traces; ++tr) {
         const double dxm = ox - P.mx[tr], dym = oy - P.my[tr];
         const double d2 = dxm * dxm + dym * dym;
-        cnt += d2 <= P.fold_d2_max;
+        const bool in_fold = d2 <= P.fold_d2_max;   // the maximum cuts for itself, also below the minimum
+        cnt += in_fold;
         const float d = (float)sqrt(d2);
-        const bool act = tv && d <= s.ap;
+        const bool act = tv && in_fold && d <= s.ap;
         if (__any_sync(0xffffffffu, act)) {
             const float dxs = (float)(ox - P.sx[tr]), dys = (float)(oy - P.sy[tr]);
             const float dxr = (float)(ox - P.rx[tr]), dyr = (float)(oy - P.ry[tr]);

@@ -108,3 +108,22 @@ def test_interpolators_cut_at_the_maximum(method, precision, cuda_kernel_factory
     got, ref = _out(), _out()
     k.migrate_tile(tb, got, vel)
     _check(tb, vel, cfg, "straight_ray", precision, got, ref)
+
+
+def test_learned_form_cuts_at_the_maximum(cuda_kernel_factory):
+    """eta = 0 and a network that answers 0: the learned traveltime is the straight one."""
+    import torch
+    from pstm_b200 import surrogate as S
+    tb, vel, cfg = _case("anisotropic_vti", max_aperture_m=300.0, min_aperture_m=500.0)
+    cfg = dataclasses.replace(cfg, vti_eta_constant=0.0)
+    k = cuda_kernel_factory(cfg)
+    ref = _out()
+    dtb, dvel, fresh = _device(tb, vel, ref)
+    got = fresh()
+    zero = S.Net(torch.zeros(S.N_PARAMS, dtype=torch.float32, device="cuda"),
+                 S.survey_domain("anisotropic_vti", h_max_m=3200.0), out_scale=0.5)
+    _, rep = k.migrate_tile_learned(dtb, got, dvel, zero, cfg, max_residual_ms=-1.0)
+    torch.cuda.synchronize()
+    assert rep["used_surrogate"]
+    got = dataclasses.replace(got, image=got.image.cpu().numpy(), fold=got.fold.cpu().numpy())
+    _check(tb, vel, cfg, "anisotropic_vti", "fp32", got, ref)
