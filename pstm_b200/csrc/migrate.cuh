@@ -262,10 +262,16 @@ __device__ __forceinline__ void point_state(const KParams &P, int p, int t, int 
         if (P.cr_k_zero) s.iv2 = ts.ivwc * ts.ivwc;   // |k| ~ 0: straight rays in v0 (curved_ray.py:35-38)
     }
     s.ap = (float)ap;
+    // x = d itw + tsn is 0 or less before the taper and 1 or more beyond the aperture; the MID
+    // loop has no other test of the aperture.  Without one only d = 0 is inside (0), or nothing
+    // is (below 0).  A hard cut has x = -1 throughout, and tests of its own.
     const float width = s.ap * P.taper_f;
-    if (width > 0.f) {
+    if (width > 1e-30f) {
         s.itw = rcp_approx(width);
         s.tsn = -(s.ap * (1.f - P.taper_f)) * s.itw;
+    } else if (P.taper_f > 0.f) {
+        s.itw = 1e30f;
+        s.tsn = s.ap < 0.f ? 1.f : 0.f;
     } else {
         s.itw = 0.f;
         s.tsn = -1.f;

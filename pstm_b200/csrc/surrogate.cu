@@ -439,8 +439,7 @@ __global__ void __launch_bounds__(128) migrate_learned_kernel(const KParams P, c
             const float a0 = amp_at<AMP>(row, i0), a1 = amp_at<AMP>(row, ok ? i0 + 1 : 0);
             const float amp = fmaf(fr, a1 - a0, a0);
             float wt = ok ? (P.w ? (float)P.w[tr] : 1.f) : 0.f;
-            const float x = fmaf(d, s.itw, s.tsn);
-            wt *= x > 0.f ? taper_weight(x) : 1.f;
+            wt *= taper_weight(__saturatef(fmaf(d, s.itw, s.tsn)));
             const float Tw = T * tw;
             const float rT = rcp_approx(Tw);
             float gw = w_two ? s.K * rT * rT : (w_one ? s.K * rT : 1.f);

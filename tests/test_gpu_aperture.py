@@ -127,3 +127,24 @@ def test_learned_form_cuts_at_the_maximum(cuda_kernel_factory):
     assert rep["used_surrogate"]
     got = dataclasses.replace(got, image=got.image.cpu().numpy(), fold=got.fold.cpu().numpy())
     _check(tb, vel, cfg, "anisotropic_vti", "fp32", got, ref)
+
+
+@pytest.mark.parametrize("taper", [0.1, 1.0, 0.0])
+@pytest.mark.parametrize("precision", ["exact", "fast", "fp32"])
+@pytest.mark.parametrize("kind,k", [("straight_ray", 0.5), ("curved_ray", 0.0), ("anisotropic_vti", 0.5)])
+def test_no_aperture_at_time_zero(kind, k, precision, taper, cuda_kernel_factory):
+    """Without a minimum the aperture of t = 0 is 0 m: only a midpoint on the pillar
+    lies inside it, at full weight, whatever the other times of its block take."""
+    from pstm_b200.base import create_trace_block
+    tb, vel, cfg = _case(kind, max_aperture_m=800.0, min_aperture_m=0.0, taper_fraction=taper, apply_obliquity=False,
+                         curved_ray_k=k)
+    sx, sy, rx, ry = (np.array(a) for a in (tb.source_x, tb.source_y, tb.receiver_x, tb.receiver_y))
+    sx[7], sy[7], rx[7], ry[7] = 20.0 - 60.0, 40.0, 20.0 + 60.0, 40.0   # midpoint on pillar (1, 2)
+    tb = create_trace_block(np.asarray(tb.amplitudes), sx, sy, rx, ry, sample_rate_ms=4.0)
+    ker = cuda_kernel_factory(cfg, precision=precision)
+    got, ref = _out(t0=0.0), _out(t0=0.0)
+    getattr(ker, METHOD[kind])(tb, got, vel)
+    _check(tb, vel, cfg, kind, precision, got, ref)
+    assert np.count_nonzero(ref.image[:, :, 0]) == 1
+    tol = 1e-5 if precision == "exact" else 1e-4
+    assert np.abs(got.image[:, :, 0] - ref.image[:, :, 0]).max() <= tol * np.abs(ref.image[1, 2, 0])
