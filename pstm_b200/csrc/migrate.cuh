@@ -135,6 +135,12 @@ __device__ __forceinline__ float scaled_double_to_float(double x) {
     return __uint_as_float(__funnelshift_l((unsigned)__double2loint(x), (unsigned)__double2hiint(x), 3));
 }
 
+// The same, rounded to the nearest float: half a unit added to the bits first, two
+// more integer instructions (the hardware's conversion takes 9 issue cycles).
+__device__ __forceinline__ float scaled_double_to_float_rn(double x) {
+    return scaled_double_to_float(__longlong_as_double(__double_as_longlong(x) + (1ll << 28)));
+}
+
 template <int AMP>
 __device__ __forceinline__ float amp_at(const unsigned char *row, int i) {
     if constexpr (AMP == AMP_F32) {
@@ -248,7 +254,7 @@ __device__ __forceinline__ void point_state(const KParams &P, int p, int t, int 
     ts.tz_in = ts.tz && s0 >= 0.0 && s0 < (double)(P.ns - 1);
     ts.vz = ts.vz2 = ts.ivwc = 0.f;
     ts.vz64 = 0.0;
-    float ivw = (float)rv;
+    double rvw = rv;   // 1/v_w
     s.iv2 = (float)(rv * rv);
     s.iv2r = s.iv2;
     s.B = rvdt * rvdt;
@@ -257,8 +263,8 @@ __device__ __forceinline__ void point_state(const KParams &P, int p, int t, int 
         ts.vz64 = P.cr_v0 + P.cr_k * z;
         ts.vz = (float)ts.vz64;
         ts.vz2 = (float)(ts.vz64 * ts.vz64);
-        ts.ivwc = (float)(1.0 / ts.vz64);
-        ivw = ts.ivwc;
+        rvw = 1.0 / ts.vz64;
+        ts.ivwc = (float)rvw;
         if (P.cr_k_zero) s.iv2 = ts.ivwc * ts.ivwc;   // |k| ~ 0: straight rays in v0 (curved_ray.py:35-38)
     }
     s.ap = (float)ap;
@@ -277,13 +283,15 @@ __device__ __forceinline__ void point_state(const KParams &P, int p, int t, int 
         s.tsn = -1.f;
     }
     // 1/(v T_sec) = ivw_t / T
+    const float ivw = (float)rvw;
     s.ivw_t = unit == UNIT_METRES ? 1.f : (unit == UNIT_SAMPLES ? ivw * P.inv_dt_f : ivw);
     s.aaA = P.aa_cA * ivw;
     s.aa_k = s.aaA * s.ivw_t;
     s.aa_thr = 0.01f * rcp_approx(unit == UNIT_SECONDS ? ivw : ivw * P.inv_dt_f);
     s.thr_s = unit == UNIT_SECONDS ? s.aa_thr * (float)P.dt_s : s.aa_thr;
-    const float Kt = P.obliquity ? (float)(t0 * ut) : 1.f;   // the obliquity's numerator
-    s.K = P.spreading ? Kt * s.ivw_t : Kt;
+    // rounded once: an error of 1/v_w would be common to a whole image in a constant velocity
+    const double Kt = P.obliquity ? t0 * ut : 1.0;   // the obliquity's numerator
+    s.K = (float)(P.spreading && unit != UNIT_METRES ? Kt * (unit == UNIT_SAMPLES ? rvw * P.inv_dt : rvw) : Kt);
     s.t02v2 = 0.f;
     s.c1 = 1.f;
     s.e2 = 0.f;
@@ -1166,8 +1174,10 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                 const double T2 = exact_time<TT, KZ, decltype(clamp_c)::value>(P, log_tab, xs[g], ts[g].tz, ts[g].tzero, B, Cd, v);
                 word = (unsigned)__double2hiint(v);
                 f = __uint_as_float(__funnelshift_r((unsigned)__double2loint(v), 0x7Fu, 9));
-                T = scaled_double_to_float(T2);
-                if constexpr (decltype(clamp_c)::value) {   // (nearest but for straight rays: these only truncate)
+                // rounded, but for straight rays truncated: 2^-24 of the weights either way round
+                if constexpr (TT == TT_STRAIGHT) T = scaled_double_to_float(T2);
+                else T = scaled_double_to_float_rn(T2);
+                if constexpr (decltype(clamp_c)::value) {
                     if constexpr (TT == TT_STRAIGHT) T_test = scaled_double_to_float(T2 * xs[g].iv);
                     else T_test = (float)((CURVED ? T2 : T2 * xs[g].iv) * (1.0 / kTimeScale));
                 }
