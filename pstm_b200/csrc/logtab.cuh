@@ -3,13 +3,16 @@
 // Table-driven, after P. T. P. Tang, "Table-driven implementation of the
 // logarithm function in IEEE floating-point arithmetic", ACM TOMS 16(4), 1990:
 // x = 2^e m, m in [1, 2); the top kLogBits bits of m's fraction pick c ~ 1/m, a
-// float, and -log c from a table; z = c m - 1, |z| <= 2^-7, and log x = e log 2 -
-// log c + log1p(z), with the Taylor polynomial of log1p through z^6 (the next term
-// is below 2^-51).  Absolute error below 2^-50 + 2^-52 |log x| for every positive
-// normal x (tests/test_log_table.py).
+// float, and -log c from a table; z = c m - 1, |z| <= 2^-8, and log x = e log 2 -
+// log c + log1p(z), with the Taylor polynomial of log1p through z^6.  The next term is
+// below 2^-58, so what is left is rounding: the table entry's and those of sums of
+// size |log x|, below 2^-53 (0.75 + 3.5 |log x|) together for every positive normal x
+// (tests/test_log_table.py).
 //
 // Why not log(): it is correct nearly to the last bit for any argument, at some
-// three times the FP64 instructions.  A curved leg's sample index needs 2^-35.
+// three times the FP64 instructions.  A curved leg's sample index needs 2^-35, and
+// the square roots in the argument are good to 2^-44.  64 entries and the same
+// polynomial (2^-50) took the same time.
 #pragma once
 #include <stdint.h>
 
@@ -23,7 +26,7 @@
 
 namespace pstm {
 
-constexpr int kLogBits = 6;
+constexpr int kLogBits = 7;
 constexpr int kLogEntries = 1 << kLogBits;
 struct alignas(16) LogEntry {
     double c, l;   // 1/m at the middle of the entry's interval, -log c

@@ -1446,10 +1446,9 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                 float4 Bf = make_float4((float)ds2, (float)dr2, 0.f, 0.f);
                 if constexpr (CURVED) {
                     const double k2 = P.cr_k2, v0 = P.cr_v0;
-                    const double bs = v0 + sqrt_newton(fma(k2, ds2, v0 * v0));
-                    const double br = v0 + sqrt_newton(fma(k2, dr2, v0 * v0));
-                    const double2 Cd = TT == TT_CURVED ? make_double2(rcp_newton(bs * br), 0.0)
-                                                       : make_double2(rcp_newton(bs), rcp_newton(br));
+                    const double bs = v0 + sqrt(v0 * v0 + k2 * ds2), br = v0 + sqrt(v0 * v0 + k2 * dr2);
+                    const double2 Cd = TT == TT_CURVED ? make_double2(1.0 / (bs * br), 0.0)
+                                                       : make_double2(1.0 / bs, 1.0 / br);
                     if constexpr (EXACT) {
                         *reinterpret_cast<double2 *>(r + RC) =
                             TT == TT_CURVED ? make_double2(0.25 * Cd.x, 0.0) : make_double2(0.5 * Cd.x, 0.5 * Cd.y);

@@ -38,3 +38,23 @@ def test_log_table_against_libm(tmp_path):
     ref = np.log(x.astype(np.longdouble))
     err = np.abs(y.astype(np.longdouble) - ref)
     assert np.all(err <= 2.0 ** -50 + 2.0 ** -52 * np.abs(ref))
+
+
+def test_log_table_is_left_with_roundings(tmp_path):
+    """No truncation error beside the roundings of a log(): z^7 / 7 with |z| <= 2^-8 +
+    2^-24 is below 2^-58; the entry's rounding is 2^-54 (|log c| < 0.7), log 2's 2.3e-17
+    per power of 2, and three sums of size |log x| + 2^-8 round by half a unit each:
+    2^-53 (0.5 + 0.21 (1 + 1.45 |log x|) + 3 |log x| + 0.04) in all."""
+    src, lib = tmp_path / "logtab.cpp", tmp_path / "logtab.so"
+    src.write_text(SRC)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(ROOT, "pstm_b200", "csrc"),
+                    "-o", str(lib), str(src)], check=True)
+    f = ctypes.CDLL(str(lib)).run
+    f.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_long]
+    edges = (1.0 + np.arange(257) / 256.0)[:, None] * (1.0 + np.array([-2.0, -1.0, 0.0, 1.0, 2.0]) * 2.0 ** -52)
+    x = np.concatenate([np.exp(np.random.default_rng(4).uniform(-9, 9, 400000)), edges.ravel()])
+    y = np.empty_like(x)
+    f(x.ctypes.data, y.ctypes.data, len(x))
+    ref = np.log(x.astype(np.longdouble))
+    err = np.abs(y.astype(np.longdouble) - ref)
+    assert np.all(err <= 2.0 ** -53 * (0.75 + 3.5 * np.abs(ref)))
