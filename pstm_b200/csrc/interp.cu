@@ -57,10 +57,11 @@ __device__ inline float rcp_r(float x) { return rcp_approx(x); }
 // f, 0 <= f < 1 (0 <= i + f < ns - 1 is checked by the caller); linear also serves
 // the wide methods within their half-width of a trace end.
 // R is the arithmetic of the weights and taps: double (exact path) or float
-// (fast path); the sample index is FP64 in both.
+// (fast path); index and fraction are FP64 in both, and so is which sample is nearest.
 template <int AMP, typename R>
-__device__ R interpolate_narrow(const unsigned char *row, int ns, int i, R f, int method) {
-    if (method == PSTM_INTERP_NEAREST) return sample_at<AMP, R>(row, f < R(0.5) ? i : i + 1);
+__device__ R interpolate_narrow(const unsigned char *row, int ns, int i, double fr, int method) {
+    if (method == PSTM_INTERP_NEAREST) return sample_at<AMP, R>(row, fr < 0.5 ? i : i + 1);
+    const R f = (R)fr;
     if (method == PSTM_INTERP_CUBIC && i >= 1 && i < ns - 2) {   // Catmull-Rom
         const R p0 = sample_at<AMP, R>(row, i - 1), p1 = sample_at<AMP, R>(row, i);
         const R p2 = sample_at<AMP, R>(row, i + 1), p3 = sample_at<AMP, R>(row, i + 2);
@@ -133,6 +134,11 @@ constexpr int taylor_last(double y) {
 // final sum; on a sample (f = 0) the sinc weights of the other taps are 0 by
 // themselves, the Lanczos weights all vanish and the sample is returned.
 //
+// The fraction comes in FP64: it decides which sample is nearest, and f - 1 is rounded
+// from it, not from f.  Next to a fraction of 1 the Lanczos tap there needs x_1 = f - 1
+// and sin(pi x_1 / HW) to their own size: its sine is a polynomial of x_1, since the
+// rotation of C and S leaves an absolute error.
+//
 // The form before this one took a Newton-refined reciprocal, a rotation of the
 // window angle and a libm sincospi per sample: 1160 issue cycles a pair for sinc8
 // in FP64 (FP64 instructions take 2.1-3.4 cycles to issue).
@@ -142,7 +148,7 @@ struct Wide {
 
     const unsigned char *row;
     int i, i_max;
-    R f, C, S, acc, norm;
+    R f, f1, C, S, S1, acc, norm;   // f1 = f - 1, S1 = sin(pi f1 / HW) (Lanczos)
     R E[HW], FE[HW];   // E[k - 1]: product of the D's but D_k; f E
 
     // C cos + S sin with compile-time factors; 0 and 1 cost nothing
@@ -156,7 +162,7 @@ struct Wide {
     template <int J>
     __device__ __forceinline__ void tap_pair(bool live) {
         if constexpr (LANCZOS) {
-            const R sn = rotate(S, C, win_cos<HW, J>, -win_sin<HW, J>);
+            const R sn = J == 1 ? S1 : rotate(S, C, win_cos<HW, J>, -win_sin<HW, J>);
             const R ea = x_over<J>(), eb = x_over<J - HW>();
             const R wa = (J & 1 ? -sn : sn) * ea * ea, wb = ((J - HW) & 1 ? sn : -sn) * eb * eb;
             add(wa, i + J);
@@ -177,7 +183,8 @@ struct Wide {
     template <int K>   // E / x_K = x_{1-K} E_k
     __device__ __forceinline__ R x_over() const {
         constexpr int k = K > 0 ? K : 1 - K;
-        return FE[k - 1] + (R)(K - 1) * E[k - 1];
+        if constexpr (K == 0) return f1 * E[0];
+        else return FE[k - 1] + (R)(K - 1) * E[k - 1];
     }
     __device__ __forceinline__ void add(R w, int j) {
         acc += sample_at<AMP, R>(row, j) * w;
@@ -187,23 +194,31 @@ struct Wide {
     __device__ __forceinline__ void taps(std::integer_sequence<int, J...>, bool live) {
         (tap_pair<J + 1>(live), ...);
     }
-    __device__ __forceinline__ R run(const unsigned char *r, int ns, int i0, R f0) {
-        if (i0 < HW || i0 >= ns - HW) return sample_at<AMP, R>(r, i0) * (R(1) - f0) + sample_at<AMP, R>(r, i0 + 1) * f0;
+    __device__ __forceinline__ R run(const unsigned char *r, int ns, int i0, double fr) {
+        if (i0 < HW || i0 >= ns - HW) {
+            const R fl = (R)fr;
+            return sample_at<AMP, R>(r, i0) * (R(1) - fl) + sample_at<AMP, R>(r, i0 + 1) * fl;
+        }
         row = r;
         i_max = ns - 1;
         i = i0;
-        f = f0;
         if constexpr (LANCZOS) {
-            if (f < R(1e-10)) return sample_at<AMP, R>(row, i);
-            if (R(1) - f < R(1e-10)) return sample_at<AMP, R>(row, i + 1);
-        } else if (f >= R(0.5)) {   // sinc counts from the nearest sample: -0.5 <= f < 0.5
+            if (fr < 1e-10) return sample_at<AMP, R>(row, i);
+            if (1.0 - fr < 1e-10) return sample_at<AMP, R>(row, i + 1);
+        } else if (fr >= 0.5) {   // sinc counts from the nearest sample: -0.5 <= f < 0.5
             i += 1;
-            f -= R(1);
+            fr -= 1.0;
         }
+        f = (R)fr;
+        f1 = (R)(fr - 1.0);
         const R y = f * (R)(kPi / HW), u = y * y;
         C = taylor_from<0, kLast, R>(u);
         S = taylor_from<1, kLast, R>(u) * y;
-        const R g = f * f - f;
+        if constexpr (LANCZOS) {
+            const R y1 = f1 * (R)(kPi / HW);
+            S1 = taylor_from<1, kLast, R>(y1 * y1) * y1;
+        }
+        const R g = f * f1;
         R D[HW];
 #pragma unroll
         for (int k = 1; k <= HW; ++k) D[k - 1] = g - (R)(k * (k - 1));
@@ -349,8 +364,8 @@ __global__ void __launch_bounds__(kInterpThreads, PSTM_INTERP_MIN_CTAS) migrate_
                 fr += 1.0;
             }
             R amp;
-            if constexpr (HW > 0) amp = Wide<AMP, HW, LANCZOS, R>().run(row, P.ns, i0, (R)fr);
-            else amp = interpolate_narrow<AMP, R>(row, P.ns, i0, (R)fr, method);
+            if constexpr (HW > 0) amp = Wide<AMP, HW, LANCZOS, R>().run(row, P.ns, i0, fr);
+            else amp = interpolate_narrow<AMP, R>(row, P.ns, i0, fr, method);
             R w = (R)S.w[j];
             if (dj > taper_start) w *= taper_weight_r((R)((dj - taper_start) * inv_taper_w));
             const R inv = R(2) * rcp_r((R)L2);
