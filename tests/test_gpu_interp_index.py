@@ -58,3 +58,15 @@ def test_fractions_beside_a_sample(method, precision, cuda_kernel_factory):
     got = _at(tr, s, method, precision, cuda_kernel_factory)
     ref = np.array([oracle.interp(tr, x, method) for x in s])
     assert np.abs(got - ref).max() <= (1e-10 if precision == "exact" else 3e-6)
+
+
+@pytest.mark.parametrize("precision", ["exact", "fast", "fp32"])
+@pytest.mark.parametrize("method", ["nearest", "sinc4", "sinc8", "sinc16", "lanczos3", "lanczos5"])
+def test_on_a_sample_the_others_do_not_count(method, precision, cuda_kernel_factory):
+    """Within 1e-10 of a sample nearest and the wide methods return it, even beside samples that
+    are not finite (the taps' weights there are 0, and 0 x NaN is NaN)."""
+    tr = _trace()
+    tr[[20, 30, 40]] = np.nan, np.inf, -np.inf
+    s = np.array([22.0, 23.0, 28.0, 32.0, 38.0, 42.0])
+    got = _at(tr, s, method, precision, cuda_kernel_factory)
+    assert np.abs(got - tr[s.astype(int)]).max() <= 1e-9
