@@ -107,14 +107,15 @@ __device__ __forceinline__ R taylor_from(R u) {
     if constexpr (N + 2 > LAST) return (R)taylor<N>;
     else return taylor_from<N + 2, LAST, R>(u) * u + (R)taylor<N>;
 }
-// Last power of y that matters: the next ones' terms are below 2^-46 (the sample
-// index's Newton step leaves 2^-40).
+// Last power of y that matters in cos and sin up to y <= pi / 2: the next term is below
+// 2^-54, half a unit in the last place of a double below 1.
 constexpr int taylor_last(double y) {
     int n = 1;
-    double t = y;
-    while (t > 0x1p-46) t *= y / ++n;
+    double next = y * y / 2;
+    while (next > 0x1p-54) next *= y / (++n + 1);
     return n;
 }
+static_assert(taylor_last(kPi / 8) == 13 && taylor_last(kPi / 3) == 18 && taylor_last(kPi / 2) == 21, "sinc8, Lanczos-3, taper");
 
 // Windowed sinc (LANCZOS false) or Lanczos (true) of half-width HW at the
 // fractional index i + f (0 <= f < 1), normalised by the sum of the weights; linear
