@@ -98,6 +98,7 @@ struct KParams {
     double cr_B0;                // 1 / (v0 dt)^2: |k| ~ 0 straight rays in v0
     double cr_k2;                // k^2
     double cr_inv_k_dt;          // kTimeScale / (k dt)
+    double cr_inv_k_unit;        // the same per kSampleUnit
     int32_t wait_iters;          // polls of one bounded mbarrier wait before it gives up
     int32_t inject_stall;        // fault injection: the first chunks' copies are never issued, so the
                                  // bounded waits for them run out (host-selected, tests only)

@@ -79,7 +79,12 @@ constexpr int kWaitIters = 1 << 20;         // default bound of every mbarrier w
 // them into floats, and the sample index plus 2^20, times the same scale, has the
 // integer index in the high word's low bits and 32 fraction bits in the low word.
 constexpr double kTimeScale = 0x1p128;
-constexpr double kQScale = 0x1p254;         // of squares: (2^128 / 2)^2, sqrt_newton_x2 doubles
+// The weights take T in units of 256 m or 128 samples, the middle of its range, so that
+// 1 / T^2 moves no amplitude far (in metres and samples it is 2^-20 to 2^-28, and
+// amplitudes below 2^-100 lost bits to it before the point's factor gave them back).
+constexpr double kMetreUnit = 256.0, kSampleUnit = 128.0;
+constexpr double kQScale = 0x1p238;         // of squares: (2^128 / 2 / kMetreUnit)^2, the legs double their roots
+static_assert(kQScale == (kTimeScale / 2 / kMetreUnit / 0x1p100) * (kTimeScale / 2 / kMetreUnit) * 0x1p100, "");
 // 2^20 in the sum, plus 2^-22: an index within 2^-22 below an integer counts as
 // that integer (the trace-end decisions are those of an index rounded to 2^-21),
 // and the fraction's float takes the 2^-22 off again
@@ -219,12 +224,13 @@ struct PtState {
 
 // The state of output point (p, t), evaluated in FP64 as
 // numba_cpu_optimized.py:378-399 does and rounded once to FP32.  `unit` is the
-// weights' unit of the traveltime T.  In metres T is v T, the sum of the legs'
+// weights' unit of the traveltime T, `per` of the base unit.  In metres T is v T, the sum of the legs'
 // effective lengths: the spreading is 1 / (v T), the obliquity t0 v / (v T) and
 // sin(theta) = minf / (v T) then need nothing of the point but t0 v.
 enum TimeUnit { UNIT_SECONDS = 0, UNIT_SAMPLES = 1, UNIT_METRES = 2 };
 template <int TT>
-__device__ __forceinline__ void point_state(const KParams &P, int p, int t, int unit, TimeState &ts, PtState &s) {
+__device__ __forceinline__ void point_state(const KParams &P, int p, int t, int unit, double per, TimeState &ts,
+                                            PtState &s) {
     const double t0 = P.ta[t] / 1000.0;
     const double v = P.vel3d ? P.vrms[(int64_t)p * P.nt + t] : P.vrms[t];
     double eta = P.eta_const;
@@ -236,8 +242,8 @@ __device__ __forceinline__ void point_state(const KParams &P, int p, int t, int 
     s.v = v;
     s.eta = eta;
     s.iv = rvdt;
-    // units of T per second
-    const double ut = unit == UNIT_METRES ? v : (unit == UNIT_SAMPLES ? P.inv_dt : 1.0);
+    // units of T per second (`per` is a power of two)
+    const double ips = 1.0 / per, ut = (unit == UNIT_METRES ? v : (unit == UNIT_SAMPLES ? P.inv_dt : 1.0)) * ips;
     // the tests of T keep samples as their unit in metres too
     const double tt = unit == UNIT_SECONDS ? 1.0 : P.inv_dt;
     // straight rays and VTI have T >= t0, so only t0 < 1.1 ms can give T <= 1 ms;
@@ -284,14 +290,14 @@ __device__ __forceinline__ void point_state(const KParams &P, int p, int t, int 
     }
     // 1/(v T_sec) = ivw_t / T
     const float ivw = (float)rvw;
-    s.ivw_t = unit == UNIT_METRES ? 1.f : (unit == UNIT_SAMPLES ? ivw * P.inv_dt_f : ivw);
+    s.ivw_t = (unit == UNIT_METRES ? 1.f : (unit == UNIT_SAMPLES ? ivw * P.inv_dt_f : ivw)) * (float)ips;
     s.aaA = P.aa_cA * ivw;
     s.aa_k = s.aaA * s.ivw_t;
     s.aa_thr = 0.01f * rcp_approx(unit == UNIT_SECONDS ? ivw : ivw * P.inv_dt_f);
     s.thr_s = unit == UNIT_SECONDS ? s.aa_thr * (float)P.dt_s : s.aa_thr;
     // rounded once: an error of 1/v_w would be common to a whole image in a constant velocity
     const double Kt = P.obliquity ? t0 * ut : 1.0;   // the obliquity's numerator
-    s.K = (float)(P.spreading && unit != UNIT_METRES ? Kt * (unit == UNIT_SAMPLES ? rvw * P.inv_dt : rvw) : Kt);
+    s.K = (float)(P.spreading ? Kt * ips * (unit == UNIT_METRES ? 1.0 : (unit == UNIT_SAMPLES ? rvw * P.inv_dt : rvw)) : Kt);
     s.t02v2 = 0.f;
     s.c1 = 1.f;
     s.e2 = 0.f;
@@ -304,7 +310,7 @@ __device__ __forceinline__ void point_state(const KParams &P, int p, int t, int 
 }
 
 // The FP64 numbers of one point that the EXACT pair loop keeps: C = (t0 v / 2)^2
-// (times kQScale, or k^2 for curved+VTI), iv = 1 / (v dt), c1 = 1 + 2 eta, e2 = 2 eta,
+// (times kQScale, or k^2 for curved+VTI), iv = kMetreUnit / (v dt), c1 = 1 + 2 eta, e2 = 2 eta,
 // 2 v(z) and v(z)^2.
 struct XState {
     double A, C, iv, c1, e2, vz, vz2;
@@ -316,7 +322,7 @@ __device__ __forceinline__ XState exact_state(const KParams &P, const TimeState 
     x.A = ts.A;
     const double vdt = s.v * P.dt_s;
     x.C = ts.A * vdt * vdt * (CURVED ? (KZ ? 1.0 : P.cr_k2) : kQScale);
-    x.iv = s.iv;
+    x.iv = s.iv * kMetreUnit;
     x.c1 = 1.0 + 2.0 * s.eta;
     x.e2 = 2.0 * s.eta;
     x.vz = 2.0 * ts.vz64;
@@ -328,8 +334,8 @@ __device__ __forceinline__ XState exact_state(const KParams &P, const TimeState 
 template <int TT, bool KZ>
 __device__ __forceinline__ double record_square(const KParams &P, double x) {
     if constexpr (TT == TT_CURVED || TT == TT_CURVED_VTI) return KZ ? x : P.cr_k2 * x;
-    // x 2^254 by the exponent (x = 0 becomes 2^-769: as good as 0 beside C)
-    return __hiloint2double(__double2hiint(x) + (254 << 20), __double2loint(x));
+    // x kQScale by the exponent (x = 0 becomes 2^-785: as good as 0 beside C)
+    return __hiloint2double(__double2hiint(x) + (238 << 20), __double2loint(x));
 }
 // Twice v + sqrt(v^2 + k^2 h^2), the numerator of a curved leg's logarithm.
 __device__ __forceinline__ double curved_numerator(const XState &x, double kx) {
@@ -344,7 +350,7 @@ __device__ __forceinline__ double curved_numerator(const XState &x, double kx) {
 // C = VTI {ds2^2, dr2^2}, curved {1/(4 bs br), 0} or curved+VTI {1/(2 bs), 1/(2 br)},
 // bs = v0 + sqrt(v0^2 + k^2 ds2).  Returns T times 2^128 in the weights' unit and puts
 // the sample index word into `v`: the sum of 2^20 + index, times 2^128.
-// Straight and VTI work in metres: a leg's effective length is sqrt(C + x) with
+// Straight and VTI work in units of kMetreUnit: a leg's effective length is sqrt(C + x) with
 // x = h^2, and with the VTI correction sqrt(C + x - 2 eta x^2 / (C + (1+2eta) x)); the
 // legs' sum times 1 / (v dt) is the index.  Against squares of times, A + x B,
 // this needs an addition instead of a three-operand FMA per leg (2.1 instead of
@@ -376,14 +382,14 @@ __device__ __forceinline__ double exact_time(const KParams &P, const LogEntry *l
         return T;
     } else if constexpr (TT == TT_CURVED) {   // |k| ~ 0: straight rays in v0 (curved_ray.py:35-38)
         if constexpr (KZ) {
-            const double T = (sqrt_newton(fma(B.x, P.cr_B0, x.A)) + sqrt_newton(fma(B.y, P.cr_B0, x.A))) * kTimeScale;
-            v = T + magic;
-            return T;
+            const double T = sqrt_newton(fma(B.x, P.cr_B0, x.A)) + sqrt_newton(fma(B.y, P.cr_B0, x.A));
+            v = fma(T, kTimeScale, magic);
+            return T * (kTimeScale / kSampleUnit);
         } else {
             double L = log_by_table(log_tab, curved_numerator(x, B.x) * curved_numerator(x, B.y) * C.x);
             if constexpr (CLAMP) L = tz ? 0.0 : L;   // depth 0: both legs are log(1) = 0
             v = fma(L, P.cr_inv_k_dt, magic);
-            return L * P.cr_inv_k_dt;
+            return L * P.cr_inv_k_unit;
         }
     } else {
         double tcs, tcr;
@@ -407,9 +413,8 @@ __device__ __forceinline__ double exact_time(const KParams &P, const LogEntry *l
         double L = fma(tcs, sqrt_newton(us), tcr * sqrt_newton(ur));
         if constexpr (CLAMP || KZ)   // t0 = 0: nothing, or (|k| ~ 0, where no point is odd) the curved legs alone
             L = tzero ? (tz ? 0.0 : tcs + tcr) : L;
-        const double unit = KZ ? kTimeScale : P.cr_inv_k_dt;
-        v = fma(L, unit, magic);
-        return L * unit;
+        v = fma(L, KZ ? kTimeScale : P.cr_inv_k_dt, magic);
+        return L * (KZ ? kTimeScale / kSampleUnit : P.cr_inv_k_unit);
     }
 }
 
@@ -747,6 +752,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
     constexpr bool CURVED = TT == TT_CURVED || TT == TT_CURVED_VTI;
     constexpr bool HAS_C = TT != TT_STRAIGHT;
     constexpr int UNIT = !EXACT ? UNIT_SECONDS : (CURVED ? UNIT_SAMPLES : UNIT_METRES);
+    constexpr double UNIT_PER = !EXACT ? 1.0 : (CURVED ? kSampleUnit : kMetreUnit);
     constexpr unsigned INDEX_BASE = EXACT ? kHiBase : kFloatBase;
     constexpr bool LOG = CURVED && EXACT && !KZ;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -840,7 +846,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
         for (int g = 0; g < 2; ++g) {
             const int t = tblk * kTimes + 32 * g + lane;
             const bool valid = t < P.nt;
-            point_state<TT>(P, p, valid ? t : P.nt - 1, UNIT, ts[g], st[g]);
+            point_state<TT>(P, p, valid ? t : P.nt - 1, UNIT, UNIT_PER, ts[g], st[g]);
             if (EXACT) xs[g] = exact_state<TT, KZ>(P, ts[g], st[g]);
             const float A = (float)ts[g].A, B = (float)st[g].B, e = (float)st[g].eta, vz = ts[g].vz;
             bool fine = A < 1e30f && B > 0.f && B < 1e30f && st[g].iv > 0.0;   // (also not NaN)
@@ -1179,7 +1185,7 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
                 else T = scaled_double_to_float_rn(T2);
                 if constexpr (decltype(clamp_c)::value) {
                     if constexpr (TT == TT_STRAIGHT) T_test = scaled_double_to_float(T2 * xs[g].iv);
-                    else T_test = (float)((CURVED ? T2 : T2 * xs[g].iv) * (1.0 / kTimeScale));
+                    else T_test = (float)(CURVED ? T2 * (kSampleUnit / kTimeScale) : T2 * xs[g].iv * (1.0 / kTimeScale));
                 }
             } else {
                 const float4 B = *reinterpret_cast<const float4 *>(r);

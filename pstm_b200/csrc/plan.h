@@ -161,6 +161,7 @@ inline KParams make_params(const pstm_traces_desc *tr, const pstm_output_desc *o
     P.cr_B0 = 1.0 / (prm->curved_v0 * prm->curved_v0 * P.dt_s * P.dt_s);
     P.cr_k2 = prm->curved_k * prm->curved_k;
     P.cr_inv_k_dt = P.cr_k_zero ? 0.0 : kTimeScale / (prm->curved_k * P.dt_s);
+    P.cr_inv_k_unit = P.cr_inv_k_dt / kSampleUnit;
     // FP32 partial sums over one chunk where the caller asks for compensated sums (an FP32
     // accumulation error of 32 instead of 128 terms, both below the pairs' own rounding:
     // images are 1.1e-7 from FP64 either way; 0.5 % of the time of offset bins)

@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(256) probe_kernel(const __grid_constant__ KPar
         const double ox = P.xg ? P.xg[p] : P.xa[ix], oy = P.yg ? P.yg[p] : P.ya[iy];
         TimeState ts;
         PtState s;
-        point_state<TT_STRAIGHT>(P, p, t, UNIT_SECONDS, ts, s);
+        point_state<TT_STRAIGHT>(P, p, t, UNIT_SECONDS, 1.0, ts, s);
         const double dxm = ox - P.mx[tr], dym = oy - P.my[tr];
         const double d2 = dxm * dxm + dym * dym;
         const bool act = d2 <= P.fold_d2_max && (float)sqrt(d2) <= s.ap;
@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(128) migrate_learned_kernel(const KParams P, c
     // the weights are in samples when the tile was prepared for the FP64
     // sample-index kernel (its exact fallback), else in seconds; T is in seconds
     const bool samples = P.exact_units != 0;
-    point_state<TT_STRAIGHT>(P, p, tc, samples ? UNIT_SAMPLES : UNIT_SECONDS, ts, s);
+    point_state<TT_STRAIGHT>(P, p, tc, samples ? UNIT_SAMPLES : UNIT_SECONDS, 1.0, ts, s);
     if (!tv) s.ap = -1.f;
     const float tw = samples ? P.inv_dt_f : 1.f;   // T in the weights' unit
     const float t0 = (float)(P.ta[tc] / 1000.0), v = 1.f / (float)(1.0 / s.v), eta = (float)s.eta;

@@ -1,9 +1,12 @@
-"""The weights' FP32 arithmetic on the exact path (GPU)."""
+"""The weights' FP32 arithmetic on the exact path (GPU): rounding and range."""
 from __future__ import annotations
+
+import dataclasses
 
 import numpy as np
 import pytest
 
+from conftest import rel_l2
 from oracle import oracle
 
 pytestmark = pytest.mark.gpu
@@ -42,3 +45,18 @@ def test_traveltime_of_the_weights_is_rounded(kind, k0, cuda_kernel_factory):
     oracle.migrate(tb, ref, vel, cfg, kind=kind)
     assert np.all(ref.image > 0)
     assert abs(np.mean(got.image / ref.image - 1.0)) <= 3e-8
+
+
+@pytest.mark.parametrize("scale", [2.0 ** -116, 2.0 ** 100])
+@pytest.mark.parametrize("kind,k0", [("straight_ray", 0.5), ("anisotropic_vti", 0.5), ("curved_ray", 0.5),
+                                     ("curved_ray", 0.0), ("curved_vti", 0.5), ("curved_vti", 0.0)])
+def test_amplitudes_near_the_ends_of_fp32(kind, k0, scale, cuda_kernel_factory):
+    """Weights of about 2^-12 leave an amplitude of 2^-116 a normal FP32 number; the
+    steps on the way to the product must not lose what the product keeps."""
+    amps = np.random.default_rng(3).standard_normal((300, 900)).astype(np.float32)
+    tb, vel, cfg, out = _case(kind, amps, k0)
+    tiny = dataclasses.replace(tb, amplitudes=(np.asarray(tb.amplitudes, np.float64) * scale).astype(np.float32))
+    got, ref = out(), out()
+    getattr(cuda_kernel_factory(cfg), METHOD[kind])(tiny, got, vel)
+    oracle.migrate(tiny, ref, vel, cfg, kind=kind)
+    assert rel_l2(got.image / scale, ref.image / scale) <= 1e-5
