@@ -1159,9 +1159,11 @@ __global__ void __launch_bounds__(kThreads, 2) gather_kernel(const __grid_consta
             }
             if (cnt == 0) break;   // the end of the traces: the consumers stop here
         }
-        // a wait that gave up: the copies in flight must land before the CTA leaves
-        if (timeout && lane == 0)
-            for (int i = max(0, j - 2); i < j; ++i)
+        // The copies in flight must land before the CTA leaves.  Of the chunks whose consumers
+        // are not known to be done these are, after a wait of this warp that gave up, the last
+        // two; and else the last one, whose consumers may have given up themselves.
+        if (lane == 0)
+            for (int i = max(0, timeout ? j - 2 : j - 1); i < j; ++i)
                 if (!(P.inject_stall && i < 2)) mbar_wait(i & 1 ? full1 : full0, (uint32_t)((i >> 1) & 1), P.wait_iters);
     } else {
         // ------------------------------------------------------------ consumers
