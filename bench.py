@@ -564,7 +564,7 @@ def measure_batched(args, world, dist, scale: int = 1, per_bin_compare: bool = T
     lognormal trace counts between 5k and 200k (about 2M), 1000 BF16 samples at
     4 ms, each bin into its own 128 x 128 x 1000 FP32 image, VTI traveltime with
     the case-2 velocity and eta(t0).  All bins in one graph-replayed
-    launch with the autotuned shape, against the same bins as one per-tile call
+    launch with the autotuned chunk depth, against the same bins as one per-tile call
     each (the reference's bin loop).  Every bin keeps 1/scale of its traces
     (the first ones); at scale 1 the full case (~2M traces, one ~100 s launch)
     is timed once and the per-bin comparison is left to a reduced run."""

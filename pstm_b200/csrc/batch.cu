@@ -1,6 +1,6 @@
 // batch.cu -- the batched form: many bins (offset or OVT gathers) that share
-// one output tile geometry, migrated by ONE persistent launch that is
-// captured in a CUDA graph, plus the autotuner of its launch shape.
+// one output tile geometry, migrated by ONE launch that is captured in a CUDA
+// graph, plus the autotuner of its traces per chunk.
 //
 // The reference migrates its gather bins one after another, each bin a
 // sequence of per-tile kernel calls (pstm/pipeline/executor.py:960-975).
@@ -48,7 +48,7 @@ struct BatchPlan {
     std::vector<BinWork> work;   // non-empty bins, most traces first
 };
 
-// Workload class of the tuned shapes.
+// Workload class of the tuned chunk depths.
 std::string class_key(const pstm_traces_desc *tr, const pstm_output_desc *out, const pstm_velocity_desc *vel,
                       const pstm_params *prm) {
     char buf[192];
@@ -93,7 +93,7 @@ int32_t check_bins(Ctx *c, const pstm_traces_desc *tr, const pstm_output_desc *o
     return PSTM_OK;
 }
 
-// Validates the arguments, picks the launch shape (forced, tuned or default),
+// Validates the arguments, picks the traces per chunk (forced, tuned or default),
 // makes sure every buffer exists and fills the plan.  Allocates; enqueues
 // nothing.  bp.work is empty when there is nothing to migrate.
 int32_t plan_batch(Ctx *c, const pstm_traces_desc *tr, const pstm_output_desc *out, const pstm_velocity_desc *vel,
@@ -176,7 +176,7 @@ int32_t enqueue_batch(Ctx *c, BatchPlan &bp, cudaStream_t st) {
 }
 
 // The arguments a captured graph depends on: every launch parameter, the work
-// list and the launch shape (the buffers of the context are inside P).
+// list and the grid (the buffers of the context are inside P).
 std::vector<unsigned char> graph_key(const BatchPlan &bp) {
     std::vector<unsigned char> k;
     auto put = [&](const void *p, size_t n) {

@@ -148,7 +148,7 @@ int32_t pstm::ctx::check_error_word(Ctx *c) {
                     "correctly and must be discarded");
     if (w & KERR_WAIT_TIMEOUT)
         return fail(c, PSTM_ERR_TIMEOUT,
-                    "a bounded wait for a trace-row copy gave up; the image and fold may hold partial sums "
+                    "a bounded wait for a chunk of traces gave up; the image and fold may hold partial sums "
                     "of this call and must be discarded");
     return PSTM_OK;
 }

@@ -73,7 +73,10 @@ constexpr int kPool = kChunk * kRowPitch;   // staged samples of one buffer
 constexpr int kMaxSplits = 8;               // CTAs of a cluster that share an item's traces
 constexpr int kFlush = 4;                   // chunks whose FP32 sums are added into FP64 together (a power of 2)
 constexpr int kFoldPillars = 8;             // pillars per fold-counting CTA
-constexpr int kWaitIters = 1 << 20;         // default bound of every mbarrier wait loop (KParams::wait_iters)
+// Default bound of every mbarrier wait loop (KParams::wait_iters), in polls that each may
+// block for a while.  A consumer's wait covers the producer's search for the next traces too:
+// one of 200 million midpoints, 2.1 s, did not exhaust it.
+constexpr int kWaitIters = 1 << 20;
 
 // EXACT path: traveltimes are carried times 2^128, so that a funnel shift turns
 // them into floats, and the sample index plus 2^20, times the same scale, has the
@@ -202,7 +205,7 @@ struct TimeState {
     float tguard;          // 1 ms in the unit of T's tests
     float vz, vz2, ivwc;   // curved: velocity at image depth, 1/vz
     bool tzero;
-    bool tz, tz_in;        // t0 = 0 with T = 0 exactly for every pair; its sample index inside the trace
+    bool tz;               // t0 = 0 with T = 0 exactly for every pair
     double A;              // (t0 / (2 dt))^2 (at least 1e-20)
     double vz64;           // curved kinds: v(z) of the image depth
 };
@@ -256,8 +259,6 @@ __device__ __forceinline__ void point_state(const KParams &P, int p, int t, int 
     ts.A = fmax(th * th, 1e-20);   // keeps the FP64 legs > 0 at t0 = 0
     ts.tzero = !(t0 > 0.0);
     ts.tz = ts.tzero && P.t0_zero_exact;
-    const double s0 = (0.0 - P.tstart_s) * P.inv_dt;
-    ts.tz_in = ts.tz && s0 >= 0.0 && s0 < (double)(P.ns - 1);
     ts.vz = ts.vz2 = ts.ivwc = 0.f;
     ts.vz64 = 0.0;
     double rvw = rv;   // 1/v_w

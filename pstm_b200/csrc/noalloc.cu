@@ -16,7 +16,7 @@
 // streams, different host threads) race for it and must be serialised by the
 // caller.
 //
-// The kernel reports device-side failures (a bounded wait for a trace-row copy
+// The kernel reports device-side failures (a bounded wait for a chunk of traces
 // that gave up) in the error word; pstm_cuda_noalloc_status reads it back once
 // the caller's stream has drained.
 #include <cuda_runtime.h>
@@ -146,7 +146,7 @@ extern "C" int32_t pstm_cuda_noalloc_status(void *stream) {
     if (e != cudaSuccess) return cuda_fail(e, "reading the allocation-free error word");
     if (w & KERR_WAIT_TIMEOUT)
         return fail(PSTM_ERR_TIMEOUT,
-                    "a bounded wait for a trace-row copy gave up in the last allocation-free call; its image "
+                    "a bounded wait for a chunk of traces gave up in the last allocation-free call; its image "
                     "and fold may hold partial sums and must be discarded");
     return PSTM_OK;
 }

@@ -505,9 +505,9 @@ class CudaKernel:
                         segment_traces: int = 0, count_items: bool = False) -> KernelMetrics:
         """Migrate an output grid with the trace-centric (scatter) schedule:
         every trace is read once for the whole grid, as in the reference's
-        trace-centric kernel (``pstm_trace_centric.metal:112-236``), with the
-        gather kernel's partial sums and one atomic add per output sample per
-        (segment, pillar block, time block) item.  ``traces`` are CUDA tensors,
+        trace-centric kernel (``pstm_trace_centric.metal:112-236``): one launch
+        whose CTAs (pillar block, time block) walk the segments that reach them
+        and add into the image once.  ``traces`` are CUDA tensors,
         best in midpoint order (``pstm_b200.spatial.sort_panel``); the output
         has a regular grid (ascending ``x_axis``, ``y_axis``).  The result is
         ``migrate_tile``'s up to the order of floating-point additions.  With
@@ -697,7 +697,7 @@ def migrate_bins(kernel: "CudaKernel", traces, bins, geometry, velocity, config=
 
 def autotune_bins(kernel: "CudaKernel", traces, bins, geometry, velocity, config=None,
                   kernel_type: str = "straight_ray", pairs_per_candidate: int = 0) -> dict:
-    """Time the candidate launch shapes of the batched form on a sample of
+    """Time the candidate depths (traces per chunk) of the batched form on a sample of
     this batch and keep the fastest in the kernel's context (later
     :func:`migrate_bins` calls of the same workload class use it)."""
     import torch
