@@ -36,7 +36,7 @@
 // pipelining, scalar instead of packed FP32, and one or three CTAs per SM instead
 // of two are all within 8 % of each other or slower.  Records cost 220 cycles a warp
 // and chunk.  64 x 64 pillars x 1500 times x 16,384 traces, 3-D velocity, AA: 191 ms
-// with whole rows staged and state reloaded from tables per chunk, 118 ms now.
+// with whole rows staged and state reloaded from tables per chunk, 120 ms now.
 //
 // Reference semantics (paths relative to the reference project):
 //   loop structure, fold, aperture, taper, weights  numba_cpu_optimized.py:147-231
